@@ -56,12 +56,12 @@ enum UnitFlags { UF_STAGE_IN = 1, UF_STAGE_OUT = 2, UF_STAGE_OUT_T = 4 };
 
 struct UnitPlan {
   PassPlan pp;
-  const Cx<float>* tw;  // W_n^k for this transform length
+  const Cx<float>* tw;  // stage-ordered twiddles of this pass plan
 };
 
 struct WorkUnit {
   PassPlan pp;                  // the unit's pass plan (a copy, so one table read fetches everything)
-  const Cx<float>* tw;          // W_n^k for the unit's transform length
+  const Cx<float>* tw;          // stage-ordered twiddles of the unit's pass plan
   long long src, dst;           // element offset of point 0 of slot 0 (data or workspace)
   long long src_slot, dst_slot;  // elements between slots
   long long src_pt, dst_pt;     // elements between points
@@ -322,6 +322,7 @@ int npad_of(int n) { return n + 1 + ((n + 1) >> 4) + 1; }
 
 bool factor_radices(int n, int maxe, std::vector<int>& radices, std::string& why);
 int get_twiddle_table(int dev, int count, int den, bool f64, void** out);
+int get_stage_table(int dev, const std::vector<int>& radices, bool f64, void** out);
 
 }  // namespace vdx
 
@@ -437,7 +438,7 @@ int vdx_batch_plan_create(const vdx_batch_item* items, int nitems, int inverse, 
     up.pp.npad = npad;
     set_pass_tables(up.pp);
     void* tw = nullptr;
-    if (get_twiddle_table(dev, n, n, false, &tw) != VDX_OK) return -4;
+    if (get_stage_table(dev, radices, false, &tw) != VDX_OK) return -4;
     up.tw = reinterpret_cast<const Cx<float>*>(tw);
     smem = std::max(smem, need(M));
     plans.push_back(up);

@@ -135,6 +135,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kC2Threads, 1) k_con
     pl.t = tid / G::MC;
     const Cx<float>* ker = a.ker + (a.ker_bs ? img * a.ker_bs : 0);
     const Cx<float>* twc = a.tw_col;
+    const Cx<float>* twcr = a.tw_colr;
     const float cs = a.col_scale;
     for (int g = rank; g < G::TILES; g += C) {
       const int c = g * G::MC + pl.m;
@@ -167,7 +168,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kC2Threads, 1) k_con
           }
         }
       });
-      Pl.template run<true, true>(v, pl, xch, twc);
+      Pl.template run<true, true>(v, pl, xch, twcr);
       Pl.template last<true>([&](auto rc) {
         constexpr int RR = decltype(rc)::value;
         each_natural<RR, MAXE, float>(v, H / RR, G::TC, pl.t, [&](int pos, Cx<float> val) {

@@ -32,11 +32,10 @@ struct PassPlan {
   int T;     // threads per transform
   int M;     // transforms (rows or columns) per CTA
   int npad;  // shared-memory slots per transform (contiguous layout)
-  // per-pass index constants of the runtime passes in forward order, set by
-  // set_pass_tables (0 = not set: the kernels derive them): the twiddle
-  // stride n / (ns R) and inv_magic(ns), ns = product of the earlier radices
-  int tws[kMaxPasses];
+  // inv_magic(ns) of each pass, ns = product of the radices run before it, in
+  // forward and in reversed pass order (set_pass_tables)
   unsigned nsm[kMaxPasses];
+  unsigned nsmr[kMaxPasses];
   unsigned tmag, mmag;  // inv_magic(T), inv_magic(M) where a kernel splits thread indices with them
 };
 
@@ -45,12 +44,12 @@ __host__ __device__ __forceinline__ unsigned inv_magic(int d) { return d > 1 ? 0
 
 // Fills the per-pass constants of a pass plan whose n and radix list are set.
 inline void set_pass_tables(PassPlan& pp) {
-  int ns = 1;
+  int ns = 1, nsr = 1;
   for (int q = 0; q < pp.npass; ++q) {
-    const int R = pp.radix[q];
-    pp.tws[q] = pp.n / (ns * R);
     pp.nsm[q] = inv_magic(ns);
-    ns *= R;
+    ns *= pp.radix[q];
+    pp.nsmr[q] = inv_magic(nsr);
+    nsr *= pp.radix[pp.npass - 1 - q];
   }
   pp.tmag = inv_magic(pp.T);
   pp.mmag = inv_magic(pp.M);
@@ -61,7 +60,10 @@ struct FftArgs {
   const void* in;
   void* out;
   const void* ker;        // convolution: kernel spectrum
-  const void* tw;         // W_n^k, k in [0, n), compute precision
+  // stage-ordered twiddles of the n-point passes (k_stage_twiddle), in the
+  // plan's pass order and, for convolutions, in reversed pass order
+  const void* tw;
+  const void* twr;
   const void* tw2;        // real transforms: W_{2n}^k, k in [0, n]
   long long ntrans;       // contiguous: number of transforms
   long long inner;        // strided: number of columns (axis stride in elements)
@@ -218,11 +220,19 @@ __device__ __forceinline__ int mod_inv(int j, int d, unsigned m) {
   return j - int(__umulhi(unsigned(j), m)) * d;
 }
 
-// RT: ns is a runtime value with nsm = inv_magic(ns) and tws = n / (ns R);
-// otherwise ns is a compile-time constant and j % ns folds
+// RT: ns is a runtime value with nsm = inv_magic(ns); otherwise ns is a
+// compile-time constant and j % ns folds.
+// tw is stage-ordered: entry k + r ns of a pass holds W_{ns R}^{k r}, so the
+// lanes of a warp (consecutive j, hence consecutive k) read neighbouring
+// entries.  A natural table W_n^i is read at k r n/(ns R) instead, a stride
+// that puts every lane on a line of its own: those L1 wavefronts, not HBM,
+// bounded the three-pass plans (32768 x 1024 points: 113.6 us from a natural
+// table, 78.8 us from a stage-ordered one, which is the copy bandwidth; the
+// 2048-point convolutions of 4096 x 1009 Bluestein rows: 123.9 -> 96.8 us
+// with their chirp launches).
 template <int R, int MAXE, bool INV, class Re, bool RT = false>
-__device__ __forceinline__ void butterflies(Cx<Re>* v, int nb, int T, int t, int ns, int n, const Cx<Re>* tw,
-                                            unsigned nsm = 0, int tws = 0) {
+__device__ __forceinline__ void butterflies(Cx<Re>* v, int nb, int T, int t, int ns, const Cx<Re>* tw,
+                                            unsigned nsm = 0) {
   constexpr int B = MAXE / R;
 #pragma unroll
   for (int b = 0; b < B; ++b) {
@@ -230,10 +240,9 @@ __device__ __forceinline__ void butterflies(Cx<Re>* v, int nb, int T, int t, int
     if (j < nb) {
       if (ns > 1) {
         const int k = RT ? mod_inv(j, ns, nsm) : j % ns;
-        const int step = k * (RT ? tws : n / (ns * R));
 #pragma unroll
         for (int r = 1; r < R; ++r) {
-          const Cx<Re> w = ldg(&tw[r * step]);
+          const Cx<Re> w = ldg(&tw[k + r * ns]);
           v[b * R + r] = INV ? cmulc(v[b * R + r], w) : cmul(v[b * R + r], w);
         }
       }
@@ -269,15 +278,11 @@ __device__ __forceinline__ void run_passes(Cx<Re>* v, const PassPlan& pp, bool r
     const int p = reversed ? P - 1 - q : q;
     const int R = pp.radix[p];
     const bool more = q + 1 < P;
-    // per-pass constants: from the plan's tables when it has them (forward
-    // order), else one division each per pass
-    const bool tab = !reversed && pp.tws[p] > 0;
-    const unsigned nsm = tab ? pp.nsm[p] : inv_magic(ns);
-    const int tws = tab ? pp.tws[p] : n / (ns * R);
+    const unsigned nsm = reversed ? pp.nsmr[q] : pp.nsm[q];
     // one radix dispatch per pass covers the butterflies and the scatter
     radix_dispatch(R, [&](auto rc) {
       constexpr int RR = decltype(rc)::value;
-      butterflies<RR, MAXE, INV, Re, true>(v, n / RR, T, t, ns, n, tw, nsm, tws);
+      butterflies<RR, MAXE, INV, Re, true>(v, n / RR, T, t, ns, tw, nsm);
       if (more) {
         xsync(warp);
         scatter<RR, MAXE, Re, true>(
@@ -356,7 +361,7 @@ struct DynPlan {
 template <int N, int T, int MAXE, bool INV, class Re, class PL, int NS, int R, int... Rest>
 __device__ __forceinline__ void chain(Cx<Re>* v, const PassPlan& pp, const PL& pl, Cx<Re>* sm, const Cx<Re>* tw) {
   constexpr bool W = WarpLocal<PL>::value && warp_sized(T);
-  butterflies<R, MAXE, INV, Re>(v, N / R, T, pl.t, NS, N, tw);
+  butterflies<R, MAXE, INV, Re>(v, N / R, T, pl.t, NS, tw);
   if constexpr (sizeof...(Rest) > 0) {
     xsync<W>();
     scatter<R, MAXE, Re>(v, N / R, T, pl.t, NS, [&](int pos, Cx<Re> val) { sm[pl.sidx(pp, pos)] = val; });
@@ -556,6 +561,7 @@ __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 3
   const Place<STRIDED> pl(a, P.T());
   Cx<Re>* sm = smem_base<Re>();
   const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
+  const Cx<Re>* twr = reinterpret_cast<const Cx<Re>*>(a.twr);
   const S* in = reinterpret_cast<const S*>(a.in) + pl.in0();
   Cx<Re> v[MAXE];
   P.assume_t(pl.t);
@@ -598,7 +604,7 @@ __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 3
       }
     }
   });
-  P.template run<true, true>(v, pl, sm, tw);
+  P.template run<true, true>(v, pl, sm, twr);
   store_output<Plan, true, S, Re>(P, pl, a, v);
 }
 
@@ -617,6 +623,7 @@ __global__ void __launch_bounds__(256, Plan::MAXE <= 8 ? 3 : 2) k_conv_pf(FftArg
   const Place<true> pl(a, P.T());
   Cx<Re>* sm = smem_base<Re>();
   const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
+  const Cx<Re>* twr = reinterpret_cast<const Cx<Re>*>(a.twr);
   const S* in = reinterpret_cast<const S*>(a.in) + pl.in0();
   const S* ker = reinterpret_cast<const S*>(a.ker) + pl.ker0();
   P.assume_t(pl.t);
@@ -657,7 +664,7 @@ __global__ void __launch_bounds__(256, Plan::MAXE <= 8 ? 3 : 2) k_conv_pf(FftArg
         v[b * RR + r] = KOP == 0 ? cmulc(v[b * RR + r], k) : cmul(v[b * RR + r], k);
       }
   });
-  P.template run<true, true>(v, pl, sm, tw);
+  P.template run<true, true>(v, pl, sm, twr);
   store_output<Plan, true, S, Re>(P, pl, a, v);
 }
 
@@ -678,6 +685,7 @@ __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 3
   const Place<STRIDED> pl(a, P.T());
   Cx<Re>* sm = smem_base<Re>();
   const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
+  const Cx<Re>* twr = reinterpret_cast<const Cx<Re>*>(a.twr);
   unsigned dyn;
   asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
   Cx<Re>* keep = sm + (dyn / sizeof(Cx<Re>) - unsigned(MAXE) * blockDim.x);
@@ -713,7 +721,7 @@ __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 3
         }
       }
     });
-    P.template run<true, true>(v, pl, sm, tw);
+    P.template run<true, true>(v, pl, sm, twr);
     store_output<Plan, true, S, Re>(P, pl, a, v, reinterpret_cast<S*>(a.out) + k * ostride);
   }
 }
@@ -905,6 +913,24 @@ __global__ void k_twiddle(Cx<Re>* tab, int count, int den) {
   // needed because k < den
   sincospi(2.0 * double(k) / double(den), &s, &c);
   tab[k] = mk<Re>(Re(c), Re(-s));
+}
+
+// Stage-ordered twiddles of a pass list: the pass that runs radix R after
+// ns points' worth of earlier radices owns entries [ns, ns R), entry
+// k + r ns = W_{ns R}^{k r} = W_n^{k r n/(ns R)} (the same integer exponent,
+// hence the same bits, as a natural table).  The ranges of all passes tile
+// [1, n); entry 0 is never read.
+template <class Re>
+__global__ void k_stage_twiddle(Cx<Re>* tab, PassPlan pp) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= pp.n) return;
+  int ns = 1, p = 0;
+  while (p + 1 < pp.npass && i >= ns * pp.radix[p]) ns *= pp.radix[p++];
+  const int r = i / ns, k = i - r * ns;
+  const long long e = (long long)k * r * (pp.n / (ns * pp.radix[p]));
+  double s, c;
+  sincospi(2.0 * double(e) / double(pp.n), &s, &c);
+  tab[i] = mk<Re>(Re(c), Re(-s));
 }
 
 // ---------------------------------------------------------------------------

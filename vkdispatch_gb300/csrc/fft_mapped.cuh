@@ -222,6 +222,7 @@ __device__ __forceinline__ void mapped_body(const FftArgs& a, const MapArgs& m) 
   const Place<STRIDED> pl(a, P.T());
   Cx<Re>* sm = smem_base<Re>();
   const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
+  const Cx<Re>* twr = reinterpret_cast<const Cx<Re>*>(a.twr);
   Cx<Re> v[MAXE];
   P.assume_t(pl.t);
   const int n = P.n();
@@ -254,7 +255,7 @@ __device__ __forceinline__ void mapped_body(const FftArgs& a, const MapArgs& m) 
         }
       }
     });
-    P.template run<true, true>(v, pl, sm, tw);
+    P.template run<true, true>(v, pl, sm, twr);
   }
   const Re s = Re(a.scale);
   P.template last<REV>([&](auto rc) {

@@ -66,6 +66,47 @@ int get_table(int dev, int count, int den, bool f64, void** out) {
   return VDX_OK;
 }
 
+// stage-ordered twiddle tables (k_stage_twiddle): one per (device, pass list,
+// precision), with the natural tables' lifetime
+std::map<std::tuple<int, std::vector<int>, bool>, void*> g_stage_tabs;
+
+int build_stage_table(int dev, const std::vector<int>& radices, bool f64, void** out) {
+  std::lock_guard<std::mutex> lock(g_tab_mu);
+  auto key = std::make_tuple(dev, radices, f64);
+  auto it = g_stage_tabs.find(key);
+  if (it != g_stage_tabs.end()) {
+    *out = it->second;
+    return VDX_OK;
+  }
+  PassPlan pp{};
+  pp.n = 1;
+  for (int r : radices) {
+    pp.radix[pp.npass++] = r;
+    pp.n *= r;
+  }
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, size_t(pp.n) * (f64 ? 16 : 8));
+  if (e != cudaSuccess) return fail(VDX_ERR_NOMEM, std::string("twiddle table allocation: ") + cudaGetErrorString(e));
+  cudaStream_t s;
+  e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e != cudaSuccess) {
+    cudaFree(p);
+    return cuda_fail(e, "twiddle stream");
+  }
+  e = launch_stage_twiddle(p, pp, f64, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaStreamDestroy(s);
+  if (e != cudaSuccess) {
+    cudaFree(p);
+    return cuda_fail(e, "twiddle table build");
+  }
+  g_stage_tabs[key] = p;
+  *out = p;
+  return VDX_OK;
+}
+
+std::vector<int> radix_list(const PassPlan& pp) { return std::vector<int>(pp.radix, pp.radix + pp.npass); }
+
 int store_of(int t) {
   switch (t) {
     case VDX_C64: return ST_C64;
@@ -148,6 +189,10 @@ bool factor_radices(int n, int maxe, std::vector<int>& radices, std::string& why
 }
 
 int get_twiddle_table(int dev, int count, int den, bool f64, void** out) { return get_table(dev, count, den, f64, out); }
+
+int get_stage_table(int dev, const std::vector<int>& radices, bool f64, void** out) {
+  return build_stage_table(dev, radices, f64, out);
+}
 
 int set_error(int code, const char* msg) { return fail(code, msg); }
 
@@ -338,8 +383,8 @@ int plan_fused_fourstep(vdx_plan* p, int N1, int N0, long long inner, long long 
   fl.strided = strided;
   fl.grid = (unsigned)grid;
   fl.smem = smem;
-  int rc = get_table(p->dev, N1, N1, false, const_cast<void**>(&fl.twA));
-  if (rc == VDX_OK) rc = get_table(p->dev, N0, N0, false, const_cast<void**>(&fl.twB));
+  int rc = build_stage_table(p->dev, radix_list(pp), false, const_cast<void**>(&fl.twA));
+  fl.twB = fl.twA;  // square split: one pass plan
   if (rc == VDX_OK) rc = get_table(p->dev, N, N, false, const_cast<void**>(&fl.twl));
   if (rc != VDX_OK) return rc;
   e = cudaMalloc(&p->ws, p->ws_bytes);
@@ -469,8 +514,14 @@ int plan_fourstep(vdx_plan* p, long long inner, long long outer, int smem_optin)
   p->blockB = dim3(ppB.T * ppB.M);
   p->smemA = size_t(std::max(N1 * ppA.M, (N1 + 1) * ppA.M)) * 8;
   p->smemB = size_t(N0) * ppB.M * 8;
-  int rc = get_table(p->dev, N1, N1, false, const_cast<void**>(&p->fsA.tw));
-  if (rc == VDX_OK) rc = get_table(p->dev, N0, N0, false, const_cast<void**>(&p->fsB.tw));
+  // the tensor-core passes read natural tables, the butterfly passes stage-ordered ones
+  auto short_table = [&](const PassPlan& pp, const void** out) {
+    void** o = const_cast<void**>(out);
+    return p->tensor_core ? get_table(p->dev, pp.n, pp.n, false, o)
+                          : build_stage_table(p->dev, radix_list(pp), false, o);
+  };
+  int rc = short_table(ppA, &p->fsA.tw);
+  if (rc == VDX_OK) rc = short_table(ppB, &p->fsB.tw);
   if (rc == VDX_OK) rc = get_table(p->dev, N, N, false, const_cast<void**>(&p->fsA.twl));
   if (rc != VDX_OK) return rc;
   p->fsA.scale = 1.f;
@@ -539,12 +590,20 @@ int plan_conv2d_real(const vdx_fft_desc& d, vdx_plan** plan) {
   c.col_scale = d.normalize ? 1.f / float(H) : 1.f;
   c.row_scale = d.normalize ? 1.f / float(W) : 1.f;
   void* t = nullptr;
-  int rc = get_table(p->dev, W / 2, W / 2, false, &t);
+  // the kernel's compile-time plans of W/2 and H points (fft_conv2d.cu)
+  std::vector<int> rrow, rcol;
+  std::string why;
+  factor_radices(W / 2, 16, rrow, why);
+  factor_radices(H, 16, rcol, why);
+  int rc = build_stage_table(p->dev, rrow, false, &t);
   c.tw_row = static_cast<const Cx<float>*>(t);
   if (rc == VDX_OK) rc = get_table(p->dev, W / 2 + 1, W, false, &t);
   c.tw2 = static_cast<const Cx<float>*>(t);
-  if (rc == VDX_OK) rc = get_table(p->dev, H, H, false, &t);
+  if (rc == VDX_OK) rc = build_stage_table(p->dev, rcol, false, &t);
   c.tw_col = static_cast<const Cx<float>*>(t);
+  std::reverse(rcol.begin(), rcol.end());
+  if (rc == VDX_OK) rc = build_stage_table(p->dev, rcol, false, &t);
+  c.tw_colr = static_cast<const Cx<float>*>(t);
   if (rc != VDX_OK) {
     delete p;
     return rc;
@@ -1030,12 +1089,16 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
   }
 
   void* tw = nullptr;
-  int rc = get_table(p->dev, n, n, f64, &tw);
+  int rc = build_stage_table(p->dev, p->radices, f64, &tw);
+  a.tw = tw;
+  if (rc == VDX_OK && is_conv) {
+    rc = build_stage_table(p->dev, std::vector<int>(p->radices.rbegin(), p->radices.rend()), f64, &tw);
+    a.twr = tw;
+  }
   if (rc != VDX_OK) {
     delete p;
     return rc;
   }
-  a.tw = tw;
   if (even_real) {
     void* tw2 = nullptr;
     rc = get_table(p->dev, n + 1, 2 * n, f64, &tw2);

@@ -51,6 +51,7 @@ template <class S, class Re>
 cudaError_t launch_dyn_real(const FftArgs& a, const Launch& l, int op);
 
 cudaError_t launch_twiddle(void* tab, int count, int den, bool f64, cudaStream_t s);
+cudaError_t launch_stage_twiddle(void* tab, const PassPlan& pp, bool f64, cudaStream_t s);
 
 // One pass of a four-step long-axis transform (fft_large.cu): tiles of M
 // adjacent columns, one pp.n-point transform per column.  Batch b of the
@@ -61,7 +62,7 @@ struct FsArgs {
   PassPlan pp;
   const void* in;
   void* out;
-  const void* tw;   // W_n^k of the short transform
+  const void* tw;   // stage-ordered twiddles of the short transform (tensor-core passes: W_n^k)
   const void* twl;  // W_N^k of the whole axis (pass A)
   long long split;
   long long in_bs1, in_bs2, out_bs1, out_bs2;
@@ -122,9 +123,10 @@ struct Conv2dArgs {
   Cx<float>* data;          // (images, H, W/2 + 1) packed RFFT rows, in place
   const Cx<float>* ker;     // kernel spectrum, (images or 1, H, W/2 + 1)
   long long ker_bs;         // elements between images' kernel spectra (0 = broadcast)
-  const Cx<float>* tw_row;  // W_{W/2}^k, k < W/2
+  const Cx<float>* tw_row;  // stage-ordered twiddles of the W/2-point rows
   const Cx<float>* tw2;     // W_W^k, k <= W/2
-  const Cx<float>* tw_col;  // W_H^k, k < H
+  const Cx<float>* tw_col;  // and of the H-point columns, in both pass orders
+  const Cx<float>* tw_colr;
   float col_scale, row_scale;
 };
 // Bluestein transforms (bluestein.cu): chirp tables w (N) and b (M), the
