@@ -65,7 +65,7 @@ struct WorkUnit {
   long long src, dst;           // element offset of point 0 of slot 0 (data or workspace)
   long long src_slot, dst_slot;  // elements between slots
   long long src_pt, dst_pt;     // elements between points
-  const Cx<float>* twl;         // UK_COLS: W_L table of the full length
+  const Cx<float>* twl;         // UK_COLS: W_L^{n2 k1} at k1 * L2 + n2
   int kind;
   int plan;
   int nslots;  // slots (transforms, columns or rows) of this tile that exist
@@ -91,37 +91,72 @@ struct BatchArgs {
   int extra_wait;        // added to every dependency count (0 unless a test injects an unmet dependency)
 };
 
-// placement of a thread inside the current unit (the interface run_passes
-// uses).  The shared-memory slot is i*ci + m*cm + (i >> 4)*cp: (M, 1, 0) for
-// strided column tiles, (1, npad, 1) for contiguous rows -- one branch-free
-// code path for every unit kind.
-struct UnitPlace {
-  int t, m;
-  int ci, cmo, cp;  // cmo = m * cm, precomputed
-  __device__ __forceinline__ int sidx(const PassPlan&, int i) const { return i * ci + cmo + (i >> 4) * cp; }
-};
-
-// Copies a tile of contiguous rows into the padded row slots of shared
-// memory: element e is point e % n of row e / n (e < M n <= 16 * 1024, so
-// the multiply-high quotient is exact).
+// Copies a tile of contiguous rows into the row slots of shared memory:
+// element e is point e % n of row e / n (e < M n <= 16 * 1024, so the
+// multiply-high quotient is exact).
 __device__ __forceinline__ void stage_rows_in(const Cx<float>* __restrict__ s0, Cx<float>* __restrict__ sm, int total,
                                            int n, int npad, unsigned nmag) {
   for (int e = threadIdx.x; e < total; e += blockDim.x) {
     const int r = int(__umulhi(unsigned(e), nmag));
     const int i = e - r * n;
-    sm[r * npad + i + (i >> 4)] = s0[e];
+    sm[r * npad + i] = s0[e];
   }
 }
 
-// One code path for every unit kind (separate inlined copies per kind exhaust
-// the 64 registers a thread has): the store multiplies by a per-point factor
-// that is the four-step twiddle W_L^{n2 k1} for UK_COLS and the output scale
-// otherwise.  UK_ROWS2 reads workspace that other CTAs wrote in this launch
-// with ordinary (L1-cached) loads: the SM has not cached those lines before,
-// because each workspace element is read by exactly one UK_ROWS2 unit, only
-// after all UK_COLS units of its item completed, and every item's workspace
-// region starts on its own 256-byte boundary, so no cache line is shared
-// between items.
+// Source and sink of a unit's transforms (generic addresses: the tile in
+// global memory, or its staged copy in shared memory).  Point offsets inside a
+// unit stay below 2^28 (n, L1, L2 <= 16384): 32-bit.
+struct UnitIn {
+  const Cx<float>* p;
+  int pt;
+  bool valid;
+  template <int R>
+  __device__ __forceinline__ void load(Cx<float>* v, int j, int nb) const {
+    const Cx<float>* q = p + j * pt;
+    const int step = nb * pt;
+#pragma unroll
+    for (int r = 0; r < R; ++r, q += step) v[r] = valid ? *q : mk<float>(0.f, 0.f);
+  }
+};
+// Column units multiply by the four-step twiddles W_L^{n2 k1} of the thread's
+// column n2, which are laid out like the column's points.
+// The sink's fields are read from the unit table when the last pass stores, so
+// they hold no registers during the passes.
+template <bool INV>
+struct UnitOut {
+  Cx<float>* data;
+  Cx<float>* ws;
+  const WorkUnit* u;
+  Cx<float>* sm;
+  int m;
+  bool valid;
+  template <int R>
+  __device__ __forceinline__ void store(const Cx<float>* v, int j, int nb) const {
+    if (!valid) return;
+    const bool cols = u->kind == UK_COLS, stg = (u->flags & (UF_STAGE_OUT | UF_STAGE_OUT_T)) != 0;
+    const int pt = stg ? 1 : int(u->dst_pt);
+    Cx<float>* q = (stg ? sm + m * u->pp.npad : (cols ? ws : data) + u->dst + m * u->dst_slot) + j * pt;
+    const int step = nb * pt;
+    if (cols) {
+      const Cx<float>* w = u->twl + u->c0 + m + j * pt;
+#pragma unroll
+      for (int r = 0; r < R; ++r, q += step, w += step) {
+        const Cx<float> f = ldg(w);
+        *q = INV ? cmulc(v[r], f) : cmul(v[r], f);
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r, q += step) *q = scale(v[r], u->scale);
+    }
+  }
+};
+
+// One code path for every unit kind.  UK_ROWS2 reads workspace that other CTAs
+// wrote in this launch with ordinary (L1-cached) loads: the SM has not cached
+// those lines before, because each workspace element is read by exactly one
+// UK_ROWS2 unit, only after all UK_COLS units of its item completed, and every
+// item's workspace region starts on its own 256-byte boundary, so no cache
+// line is shared between items.
 template <bool INV>
 __device__ __forceinline__ void run_unit(const BatchArgs& a, const WorkUnit* __restrict__ pu, int kind,
                                          Cx<float>* sm) {
@@ -130,98 +165,57 @@ __device__ __forceinline__ void run_unit(const BatchArgs& a, const WorkUnit* __r
   // global loads the compiler may repeat instead of holding them in registers
   const WorkUnit& wu = *pu;
   const PassPlan& pp = wu.pp;
-  const Cx<float>* tw = wu.tw;
   const int n = pp.n, T = pp.T, M = pp.M;
   const bool cols = kind == UK_COLS;
-  UnitPlace pl;
   const int tid = threadIdx.x;
-  // thread index split by the plan's multiply-high reciprocals (tid < 1024)
+  // thread index split by the plan's multiply-high reciprocals (tid < 1024);
+  // slots: (M, no padding) for strided column tiles, (1, the plan's padding)
+  // for rows
+  int t, m;
+  Slots<float, false> x;
   if (cols) {
-    pl.t = M > 1 ? int(__umulhi(unsigned(tid), pp.mmag)) : tid;
-    pl.m = tid - pl.t * M;
-    pl.ci = M;
-    pl.cmo = pl.m;
-    pl.cp = 0;
+    t = M > 1 ? int(__umulhi(unsigned(tid), pp.mmag)) : tid;
+    m = tid - t * M;
+    x = Slots<float, false>{sm + m, M, 0};
   } else {
-    pl.m = T > 1 ? int(__umulhi(unsigned(tid), pp.tmag)) : tid;
-    pl.t = tid - pl.m * T;
-    pl.ci = 1;
-    pl.cmo = pl.m * pp.npad;
-    pl.cp = 1;
+    m = T > 1 ? int(__umulhi(unsigned(tid), pp.tmag)) : tid;
+    t = tid - m * T;
+    x = Slots<float, false>{sm + m * pp.npad, 1, pp.pad};
   }
-  const bool active = pl.t < T && pl.m < M;
-  if (!active) pl.t = 1 << 20;  // every butterfly index of an idle thread is out of range
-  const bool valid = active && pl.m < wu.nslots;
+  const bool active = t < T && m < M;
+  if (!active) t = 1 << 20;  // every butterfly index of an idle thread is out of range
+  const bool valid = active && m < wu.nslots;
   const int flags = wu.flags;
-  // the first pass gathers point pos of slot m from src + pos * pt +
-  // (pos >> 4) * pad: the tile in global memory, or the copy the kernel loop
-  // staged into the padded row slots of shared memory (UF_STAGE_IN).  One
-  // generic-address load path: a branch between two gathers here, or a
-  // barrier inside this function, costs the kernel 400 more bytes of spills.
-  const bool stg = (flags & UF_STAGE_IN) != 0;
-  const Cx<float>* src = stg ? sm + pl.m * pp.npad : (kind == UK_ROWS2 ? a.ws : a.data) + wu.src + pl.m * wu.src_slot;
-  // point offsets inside a unit stay below 2^28 (n, L1, L2 <= 16384): 32-bit
-  const int src_pt = stg ? 1 : int(wu.src_pt);
-  const int pad = stg ? 1 : 0;
-  Cx<float> v[MAXE];
-  radix_dispatch(pp.radix[0], [&](auto rc) {
-    constexpr int RR = decltype(rc)::value;
-    gather<RR, MAXE, float>(v, n / RR, T, pl.t, [&](int pos) {
-      if (!valid) return mk<float>(0.f, 0.f);
-      return src[pos * src_pt + (pos >> 4) * pad];
-    });
-  });
-  // row units keep each transform inside one warp when T divides 32
-  run_passes<MAXE, INV>(v, pp, false, pl, sm, tw, !cols && warp_sized(T));
-  const float sc = wu.scale;
-  if (flags & (UF_STAGE_OUT | UF_STAGE_OUT_T)) {
-    __syncthreads();  // every thread's last gather from sm is done
-    radix_dispatch(pp.radix[pp.npass - 1], [&](auto rc) {
-      constexpr int RR = decltype(rc)::value;
-      each_natural<RR, MAXE, float>(v, n / RR, T, pl.t,
-                                    [&](int pos, Cx<float> val) { sm[pl.sidx(pp, pos)] = scale(val, sc); });
-    });
-    __syncthreads();
-    Cx<float>* d0 = a.data + wu.dst;
-    const int ns = wu.nslots, total = ns * n, npad = pp.npad;
-    if (flags & UF_STAGE_OUT) {
-      const unsigned nmag = wu.nmag;
-      for (int e = tid; e < total; e += blockDim.x) {
-        const int r = int(__umulhi(unsigned(e), nmag));
-        const int i = e - r * n;
-        d0[e] = sm[r * npad + i + (i >> 4)];
-      }
-    } else {
-      // point k of row r goes to d0[r + k * dst_pt]; rows fastest across lanes
-      const unsigned smag = wu.smag;
-      const int dpt = int(wu.dst_pt);
-      for (int e = tid; e < total; e += blockDim.x) {
-        const int k = ns > 1 ? int(__umulhi(unsigned(e), smag)) : e;
-        const int r = e - k * ns;
-        d0[r + k * dpt] = sm[r * npad + k + (k >> 4)];
-      }
+  const bool stg_in = (flags & UF_STAGE_IN) != 0, stg_out = (flags & (UF_STAGE_OUT | UF_STAGE_OUT_T)) != 0;
+  UnitIn in;
+  in.p = stg_in ? sm + m * pp.npad : (kind == UK_ROWS2 ? a.ws : a.data) + wu.src + m * wu.src_slot;
+  in.pt = stg_in ? 1 : int(wu.src_pt);
+  in.valid = valid;
+  const UnitOut<INV> out{a.data, a.ws, pu, sm, m, valid};
+  // row units keep each transform inside one warp when T divides 32; a staged
+  // one-pass tile still reads and writes the thread's own row only
+  runtime_transform<MAXE, INV>(pp, t, x, wu.tw, in, out, stg_in, stg_out, !cols && warp_sized(T));
+  if (!stg_out) return;
+  __syncthreads();
+  Cx<float>* d0 = a.data + wu.dst;
+  const int ns = wu.nslots, total = ns * n, npad = pp.npad;
+  if (flags & UF_STAGE_OUT) {
+    const unsigned nmag = wu.nmag;
+    for (int e = tid; e < total; e += blockDim.x) {
+      const int r = int(__umulhi(unsigned(e), nmag));
+      const int i = e - r * n;
+      d0[e] = sm[r * npad + i];
     }
-    return;
+  } else {
+    // point k of row r goes to d0[r + k * dst_pt]; rows fastest across lanes
+    const unsigned smag = wu.smag;
+    const int dpt = int(wu.dst_pt);
+    for (int e = tid; e < total; e += blockDim.x) {
+      const int k = ns > 1 ? int(__umulhi(unsigned(e), smag)) : e;
+      const int r = e - k * ns;
+      d0[r + k * dpt] = sm[r * npad + k];
+    }
   }
-  Cx<float>* dst = (kind == UK_COLS ? a.ws : a.data) + wu.dst + pl.m * wu.dst_slot;
-  const int dst_pt = int(wu.dst_pt);
-  const bool twiddle = cols;
-  const Cx<float>* twl = wu.twl;
-  const int twstep = twiddle ? wu.c0 + pl.m : 0;  // n2; n2 * k1 < L <= 2^24
-  radix_dispatch(pp.radix[pp.npass - 1], [&](auto rc) {
-    constexpr int RR = decltype(rc)::value;
-    each_natural<RR, MAXE, float>(v, n / RR, T, pl.t, [&](int pos, Cx<float> val) {
-      if (!valid) return;
-      if (twiddle) {
-        // W_L^{n2 k1} with n2 = column, k1 = pos (n2 k1 < L)
-        const Cx<float> w = ldg(twl + twstep * pos);
-        val = INV ? cmulc(val, w) : cmul(val, w);
-      } else {
-        val = scale(val, sc);
-      }
-      dst[pos * dst_pt] = val;
-    });
-  });
 }
 
 // THREADS per CTA, MINB resident CTAs per SM (64 registers per thread).
@@ -320,8 +314,8 @@ int npad_of(int n) { return n + 1 + ((n + 1) >> 4) + 1; }
 
 }  // namespace
 
-bool factor_radices(int n, int maxe, std::vector<int>& radices, std::string& why);
-int get_twiddle_table(int dev, int count, int den, bool f64, void** out);
+bool factor_radices(int n, int maxe, std::vector<int>& radices, std::string& why, int tmax);
+int get_cross_table(int dev, int N1, int N0, void** out);
 int get_stage_table(int dev, const std::vector<int>& radices, bool f64, void** out);
 
 }  // namespace vdx
@@ -365,8 +359,8 @@ bool split_long(int L, int cta, int& L1, int& L2) {
     if (e > 16384) continue;
     std::vector<int> r;
     std::string why;
-    if (!factor_radices(d, 16, r, why) || threads_for(r, d) > cta) continue;
-    if (!factor_radices(e, 16, r, why) || threads_for(r, e) > cta) continue;
+    if (!factor_radices(d, 16, r, why, cta) || threads_for(r, d) > cta) continue;
+    if (!factor_radices(e, 16, r, why, cta) || threads_for(r, e) > cta) continue;
     if (best < 0 || std::abs(std::log((double)d) - 0.5 * std::log((double)L)) <
                         std::abs(std::log((double)best) - 0.5 * std::log((double)L)))
       best = d;
@@ -418,7 +412,7 @@ int vdx_batch_plan_create(const vdx_batch_item* items, int nitems, int inverse, 
     auto it = plan_index.find(key);
     if (it != plan_index.end()) return it->second;
     std::vector<int> radices;
-    if (!factor_radices(n, 16, radices, why)) return -1;
+    if (!factor_radices(n, 16, radices, why, cta)) return -1;
     const int T = threads_for(radices, n);
     if (T > cta) return -2;
     int M = std::max(1, cta / T);
@@ -458,7 +452,7 @@ int vdx_batch_plan_create(const vdx_batch_item* items, int nitems, int inverse, 
     const int L = it.length;
     const float scale = (inverse && normalize) ? 1.0f / float(L) : 1.0f;
     std::vector<int> r;
-    bool single = L <= 16384 && factor_radices(L, 16, r, why) && threads_for(r, L) <= cta &&
+    bool single = L <= 16384 && factor_radices(L, 16, r, why, cta) && threads_for(r, L) <= cta &&
                   size_t(npad_of(L)) * 8 + 1024 <= size_t(smem_cap);
     if (single) {
       const int p = get_plan(L, false, it.count);
@@ -493,7 +487,7 @@ int vdx_batch_plan_create(const vdx_batch_item* items, int nitems, int inverse, 
     const int pr = get_plan(L2, false, L1);
     if (pc < 0 || pr < 0) return set_error(VDX_ERR_UNSUPPORTED, ("length " + std::to_string(L) + ": " + why).c_str());
     void* twl = nullptr;
-    if (get_twiddle_table(dev, L, L, false, &twl) != VDX_OK) return VDX_ERR_NOMEM;
+    if (get_cross_table(dev, L1, L2, &twl) != VDX_OK) return VDX_ERR_NOMEM;
     const int item = nlarge++;
     const long long wsoff = (ws_elems + 31) & ~31ll;  // 256-byte aligned region per item
     ws_elems = wsoff + (long long)L * it.count;

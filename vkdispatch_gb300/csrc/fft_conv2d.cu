@@ -55,13 +55,16 @@ struct C2Geo {
 struct RowPl {  // contiguous rows: t = thread of the row, m = row of the round
   int t, m;
   int npad;
+  static constexpr bool kLinear = false;
   __device__ __forceinline__ int sidx(const PassPlan&, int i) const { return m * npad + i + (i >> 4); }
   __device__ __forceinline__ int sidx_plain(int i) const { return m * npad + i; }
 };
 
 struct ColPl {  // column tile: m = column of the tile, t = thread of the column
   int t, m, M;
+  static constexpr bool kLinear = true;
   __device__ __forceinline__ int sidx(const PassPlan&, int i) const { return i * M + m; }
+  __device__ __forceinline__ int pitch(const PassPlan&) const { return M; }
 };
 
 template <int H, int W, int C, int KOP>

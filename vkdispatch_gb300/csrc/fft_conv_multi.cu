@@ -8,7 +8,7 @@ namespace {
 
 template <class S, class Re, bool STRIDED>
 cudaError_t launch_multi(const FftArgs& a, const Launch& l, int kop, int K, long long kstride, long long ostride) {
-  using Plan = DynPlan<MaxE<Re>::value>;
+  using Plan = DynConvPlanOf<S, Re>;
   if (kop == 0) return enqueue(k_conv_multi<Plan, STRIDED, S, Re, 0>, l, a, K, kstride, ostride);
   return enqueue(k_conv_multi<Plan, STRIDED, S, Re, 1>, l, a, K, kstride, ostride);
 }

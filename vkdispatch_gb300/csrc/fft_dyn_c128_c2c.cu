@@ -4,6 +4,6 @@
 namespace vdx {
 template <>
 cudaError_t launch_dyn_c2c<Cx<double>, double>(const FftArgs& a, const Launch& l, int op, bool strided, int variant) {
-  return launch_c2c_any<DynPlan<MaxE<double>::value>, Cx<double>, double>(a, l, op, strided, variant);
+  return launch_c2c_any<DynPlanOf<Cx<double>, double>, Cx<double>, double>(a, l, op, strided, variant);
 }
 }  // namespace vdx

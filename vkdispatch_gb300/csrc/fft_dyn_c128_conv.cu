@@ -5,6 +5,6 @@ namespace vdx {
 template <>
 cudaError_t launch_dyn_conv<Cx<double>, double>(const FftArgs& a, const Launch& l, bool strided, int kop, int variant) {
   if (kop != 0) return cudaErrorInvalidValue;
-  return launch_conv<DynPlan<MaxE<double>::value>, 0, Cx<double>, double>(a, l, strided, variant);
+  return launch_conv<DynConvPlanOf<Cx<double>, double>, 0, Cx<double>, double>(a, l, strided, variant);
 }
 }  // namespace vdx

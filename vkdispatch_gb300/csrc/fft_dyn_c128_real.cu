@@ -4,6 +4,6 @@
 namespace vdx {
 template <>
 cudaError_t launch_dyn_real<Cx<double>, double>(const FftArgs& a, const Launch& l, int op) {
-  return launch_real<DynPlan<MaxE<double>::value>, Cx<double>, double>(a, l, op, true);
+  return launch_real<DynPlanOf<Cx<double>, double>, Cx<double>, double>(a, l, op, true);
 }
 }  // namespace vdx

@@ -4,6 +4,6 @@
 namespace vdx {
 template <>
 cudaError_t launch_dyn_real<c32s, float>(const FftArgs& a, const Launch& l, int op) {
-  return launch_real<DynPlan<MaxE<float>::value>, c32s, float>(a, l, op, true);
+  return launch_real<DynPlanOf<c32s, float>, c32s, float>(a, l, op, true);
 }
 }  // namespace vdx

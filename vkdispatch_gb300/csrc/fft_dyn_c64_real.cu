@@ -4,6 +4,6 @@
 namespace vdx {
 template <>
 cudaError_t launch_dyn_real<Cx<float>, float>(const FftArgs& a, const Launch& l, int op) {
-  return launch_real<DynPlan<MaxE<float>::value>, Cx<float>, float>(a, l, op, true);
+  return launch_real<DynPlanOf<Cx<float>, float>, Cx<float>, float>(a, l, op, true);
 }
 }  // namespace vdx

@@ -98,7 +98,9 @@ struct FusedArgs {
 
 struct TilePlace {
   int t, m, M;
+  static constexpr bool kLinear = true;
   __device__ __forceinline__ int sidx(const PassPlan&, int i) const { return i * M + m; }
+  __device__ __forceinline__ int pitch(const PassPlan&) const { return M; }
 };
 
 // One tile: M columns x n points.  Point pos of column m is read at

@@ -32,10 +32,12 @@ struct PassPlan {
   int T;     // threads per transform
   int M;     // transforms (rows or columns) per CTA
   int npad;  // shared-memory slots per transform (contiguous layout)
+  int pad;   // rows of a runtime plan pad one slot every 16 (see Slots)
   // inv_magic(ns) of each pass, ns = product of the radices run before it, in
   // forward and in reversed pass order (set_pass_tables)
   unsigned nsm[kMaxPasses];
   unsigned nsmr[kMaxPasses];
+  int nb[kMaxPasses];  // n / radix[p]: butterflies of the pass
   unsigned tmag, mmag;  // inv_magic(T), inv_magic(M) where a kernel splits thread indices with them
 };
 
@@ -49,8 +51,15 @@ inline void set_pass_tables(PassPlan& pp) {
     pp.nsm[q] = inv_magic(ns);
     ns *= pp.radix[q];
     pp.nsmr[q] = inv_magic(nsr);
+    pp.nb[q] = pp.n / pp.radix[q];
     nsr *= pp.radix[pp.npass - 1 - q];
   }
+  // rows pad where stepping through padded slots stays exact: every radix but
+  // the last is 16, so points are 1 apart inside a block of 16 or a multiple of
+  // 16 apart
+  pp.pad = pp.npass > 1;
+  for (int q = 0; q + 1 < pp.npass; ++q)
+    if (pp.radix[q] != 16) pp.pad = 0;
   pp.tmag = inv_magic(pp.T);
   pp.mmag = inv_magic(pp.M);
 }
@@ -89,8 +98,14 @@ struct FftArgs {
 // ---------------------------------------------------------------------------
 // thread placement
 // ---------------------------------------------------------------------------
-template <bool STRIDED>
+// PAD: rows pad one shared-memory slot every 16, which spreads the stride-R
+// scatters of power-of-two radices over the banks.  Unpadded rows (and column
+// tiles) have a linear slot layout, one addition per access instead of three
+// operations; the planner puts an odd radix first, whose scatter does not
+// conflict without padding.
+template <bool STRIDED, bool PAD = true>
 struct Place {
+  static constexpr bool kLinear = STRIDED || !PAD;
   int t, m;
   bool valid;
   bool tile_full;  // every transform slot of this CTA exists (uniform per CTA)
@@ -124,12 +139,14 @@ struct Place {
   __device__ __forceinline__ long long in0() const { return off(a.in_bs); }
   __device__ __forceinline__ long long out0() const { return off(a.out_bs); }
   __device__ __forceinline__ long long ker0() const { return off(a.ker_bs); }
-  // shared-memory slot of point i of this thread's transform; padded by one
-  // slot every 16 so the stride-R scatters of the passes do not bank-conflict
+  // shared-memory slot of point i of this thread's transform
   __device__ __forceinline__ int sidx(const PassPlan& pp, int i) const {
     if (STRIDED) return i * pp.M + m;
-    return m * pp.npad + i + (i >> 4);
+    return PAD ? m * pp.npad + i + (i >> 4) : m * pp.npad + i;
   }
+  // slots between neighbouring points of a linear layout
+  __device__ __forceinline__ int pitch(const PassPlan& pp) const { return STRIDED ? pp.M : 1; }
+  __device__ __forceinline__ int pad(const PassPlan& pp) const { return STRIDED ? 0 : pp.pad; }
   // unpadded slot, for exchanges whose accesses are unit-stride in either
   // direction (the mirrored k / n-k accesses of the real transforms)
   __device__ __forceinline__ int sidx_plain(const PassPlan& pp, int i) const {
@@ -144,8 +161,8 @@ struct Place {
 // synchronisation.  Strided column tiles spread a transform over warps.
 template <class PL>
 struct WarpLocal : FalseT {};
-template <>
-struct WarpLocal<Place<false>> : TrueT {};
+template <bool PAD>
+struct WarpLocal<Place<false, PAD>> : TrueT {};
 
 __host__ __device__ constexpr bool warp_sized(int T) { return T >= 1 && T <= 32 && 32 % T == 0; }
 
@@ -172,11 +189,16 @@ __device__ __forceinline__ void radix_dispatch(int R, F&& f) {
     case 3: f(IC<3>{}); break;
     case 4: f(IC<4>{}); break;
     case 5: f(IC<5>{}); break;
+    case 6: f(IC<6>{}); break;
     case 7: f(IC<7>{}); break;
     case 8: f(IC<8>{}); break;
     case 9: f(IC<9>{}); break;
+    case 10: f(IC<10>{}); break;
     case 11: f(IC<11>{}); break;
+    case 12: f(IC<12>{}); break;
     case 13: f(IC<13>{}); break;
+    case 14: f(IC<14>{}); break;
+    case 15: f(IC<15>{}); break;
     case 16: f(IC<16>{}); break;
     default: break;
   }
@@ -302,6 +324,455 @@ __device__ __forceinline__ void run_passes(Cx<Re>* v, const PassPlan& pp, bool r
 }
 
 // ---------------------------------------------------------------------------
+// sources and sinks of a transform.  Both see whole butterflies: a source
+// loads the R inputs, a sink stores the R outputs, of butterfly j, which sit at
+// points j + r*nb; the address steps by one precomputed stride, so a strided
+// axis costs one 64-bit addition per point rather than a 64-bit product.
+// ---------------------------------------------------------------------------
+// complex input in global memory (signal-range masked).  CTAs whose slots all
+// exist and whose range is the whole axis take the unpredicated path.
+template <class S, class Re>
+struct GlobalIn {
+  const S* p;     // point 0 of the thread's transform
+  long long ps;   // elements between points
+  int lo, hi;     // points outside [lo, hi) read as zero
+  bool full, valid;
+  template <class PL>
+  __device__ __forceinline__ GlobalIn(const FftArgs& a, const PL& pl, int n)
+      : p(reinterpret_cast<const S*>(a.in) + pl.in0()), ps(pl.ps), lo(a.sig_lo), hi(a.sig_hi),
+        full(pl.tile_full && a.sig_lo <= 0 && a.sig_hi >= n), valid(pl.valid) {}
+  template <int R>
+  __device__ __forceinline__ void load(Cx<Re>* v, int j, int nb) const {
+    const S* q = p + j * ps;
+    const long long step = nb * ps;
+    if (full) {
+#pragma unroll
+      for (int r = 0; r < R; ++r, q += step) v[r] = Conv<S, Re>::ld(q);
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r, q += step) {
+        const int pos = j + r * nb;
+        v[r] = valid && pos >= lo && pos < hi ? Conv<S, Re>::ld(q) : mk<Re>(Re(0), Re(0));
+      }
+    }
+  }
+};
+
+// GlobalIn times in_weight[element] * in_weight_scale
+template <class S, class Re>
+struct WeightedIn {
+  GlobalIn<S, Re> in;
+  const float* w;
+  Re f;
+  bool ok;
+  template <class PL>
+  __device__ __forceinline__ WeightedIn(const FftArgs& a, const PL& pl, int n)
+      : in(a, pl, n), w(a.in_weight + pl.in0()),
+        f(Re(a.in_weight_scale) * (a.in_weight_scale_ptr ? Re(__ldg(a.in_weight_scale_ptr)) : Re(1))),
+        ok(pl.tile_full || pl.valid) {}
+  template <int R>
+  __device__ __forceinline__ void load(Cx<Re>* v, int j, int nb) const {
+    in.template load<R>(v, j, nb);
+    const float* q = w + j * in.ps;
+    const long long step = nb * in.ps;
+#pragma unroll
+    for (int r = 0; r < R; ++r, q += step) v[r] = scale(v[r], ok ? Re(__ldg(q)) * f : Re(0));
+  }
+};
+
+// natural-order points in shared memory
+template <class Re>
+struct SharedIn {
+  const Cx<Re>* p;
+  template <int R>
+  __device__ __forceinline__ void load(Cx<Re>* v, int j, int nb) const {
+    const Cx<Re>* q = p + j;
+#pragma unroll
+    for (int r = 0; r < R; ++r, q += nb) v[r] = *q;
+  }
+};
+template <class Re>
+struct SharedOut {
+  Cx<Re>* p;
+  template <int R>
+  __device__ __forceinline__ void store(const Cx<Re>* v, int j, int nb) const {
+    Cx<Re>* q = p + j;
+#pragma unroll
+    for (int r = 0; r < R; ++r, q += nb) *q = v[r];
+  }
+};
+
+// scaled store to global memory (a.out unless `base` is given)
+template <class S, class Re>
+struct GlobalOut {
+  S* p;
+  long long ps;
+  Re s;
+  bool ok;
+  template <class PL>
+  __device__ __forceinline__ GlobalOut(const FftArgs& a, const PL& pl, S* base = nullptr)
+      : p((base ? base : reinterpret_cast<S*>(a.out)) + pl.out0()), ps(pl.ps), s(Re(a.scale)),
+        ok(pl.tile_full || pl.valid) {}
+  template <int R>
+  __device__ __forceinline__ void store(const Cx<Re>* v, int j, int nb) const {
+    if (!ok) return;
+    S* q = p + j * ps;
+    const long long step = nb * ps;
+#pragma unroll
+    for (int r = 0; r < R; ++r, q += step) Conv<S, Re>::st(q, scale(v[r], s));
+  }
+};
+
+// GlobalOut plus acc += loss_weight[element] * |output|^2
+template <class S, class Re>
+struct LossOut {
+  GlobalOut<S, Re> out;
+  const float* w;
+  float* acc;
+  template <class PL>
+  __device__ __forceinline__ LossOut(const FftArgs& a, const PL& pl, float* sum)
+      : out(a, pl), w(a.loss_weight + pl.out0()), acc(sum) {}
+  template <int R>
+  __device__ __forceinline__ void store(const Cx<Re>* v, int j, int nb) const {
+    if (!out.ok) return;
+    float lw[R];
+    const float* q = w + j * out.ps;
+    const long long step = nb * out.ps;
+#pragma unroll
+    for (int r = 0; r < R; ++r, q += step) lw[r] = __ldg(q);
+    out.template store<R>(v, j, nb);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const Cx<Re> y = scale(v[r], out.s);
+      *acc += lw[r] * float(y.x * y.x + y.y * y.y);
+    }
+  }
+};
+
+// the spectrum operation of a convolution, applied to the R natural-order
+// spectrum points of one butterfly.  KOP 0 multiplies by conj(kernel), 1 by
+// kernel; SPEC 1 also writes the forward spectrum to spec_out, SPEC 2 writes
+// spec_aux * conj(spectrum) * spec_scale.
+template <class S, class K, class Re, int KOP, int SPEC>
+struct SpectrumOp {
+  const K* ker;
+  S* so;
+  const S* sa;
+  Re ss;
+  long long ps;
+  bool ok;
+  template <class PL>
+  __device__ __forceinline__ SpectrumOp(const FftArgs& a, const PL& pl)
+      : ker(reinterpret_cast<const K*>(a.ker) + pl.ker0()), so(reinterpret_cast<S*>(a.spec_out) + pl.out0()),
+        sa(reinterpret_cast<const S*>(a.spec_aux) + pl.out0()), ss(Re(a.spec_scale)), ps(pl.ps),
+        ok(pl.tile_full || pl.valid) {}
+  template <int R>
+  __device__ __forceinline__ void apply(Cx<Re>* v, int j, int nb) const {
+    const long long step = nb * ps;
+    if constexpr (SPEC == 1) {
+      if (ok) {
+        S* q = so + j * ps;
+#pragma unroll
+        for (int r = 0; r < R; ++r, q += step) Conv<S, Re>::st(q, v[r]);
+      }
+    }
+    if constexpr (SPEC == 2) {
+      if (ok) {
+        S* q = so + j * ps;
+        const S* x = sa + j * ps;
+#pragma unroll
+        for (int r = 0; r < R; ++r, q += step, x += step)
+          Conv<S, Re>::st(q, scale(cmulc(Conv<S, Re>::ld(x), v[r]), ss));
+      }
+    }
+    const K* q = ker + j * ps;
+#pragma unroll
+    for (int r = 0; r < R; ++r, q += step) {
+      const Cx<Re> k = ok ? Conv<K, Re>::ld(q) : mk<Re>(Re(0), Re(0));
+      v[r] = KOP == 0 ? cmulc(v[r], k) : cmul(v[r], k);
+    }
+  }
+};
+
+// f(b, j) for the thread's butterflies j = t + b*T < nb of a pass, b a
+// compile-time constant (so that the values' register array is never indexed
+// by a loop counter)
+template <int R, int MAXE, int B = 0, class F>
+__device__ __forceinline__ void each_butterfly(int nb, int T, int t, F&& f) {
+  if constexpr (B < MAXE / R) {
+    const int j = t + B * T;
+    if (j < nb) f(IntConst<int, B>{}, j);
+    each_butterfly<R, MAXE, B + 1>(nb, T, t, f);
+  }
+}
+
+// The exchange between two passes: the R values at points i0 + r*di of the
+// transform in shared memory.  Placements with a linear slot layout step by
+// one stride; the padded row layout computes each slot.
+template <int R, class PL, class Re>
+__device__ __forceinline__ void xload(Cx<Re>* v, const Cx<Re>* sm, const PassPlan& pp, const PL& pl, int i0, int di) {
+  if constexpr (PL::kLinear) {
+    const Cx<Re>* q = sm + pl.sidx(pp, i0);
+    const int step = di * pl.pitch(pp);
+#pragma unroll
+    for (int r = 0; r < R; ++r, q += step) v[r] = *q;
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = sm[pl.sidx(pp, i0 + r * di)];
+  }
+}
+template <int R, class PL, class Re>
+__device__ __forceinline__ void xstore(const Cx<Re>* v, Cx<Re>* sm, const PassPlan& pp, const PL& pl, int i0, int di) {
+  if constexpr (PL::kLinear) {
+    Cx<Re>* q = sm + pl.sidx(pp, i0);
+    const int step = di * pl.pitch(pp);
+#pragma unroll
+    for (int r = 0; r < R; ++r, q += step) *q = v[r];
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; ++r) sm[pl.sidx(pp, i0 + r * di)] = v[r];
+  }
+}
+
+// v <- v * W_{ns R}^{k r}, then the radix-R butterfly
+template <int R, bool INV, class Re>
+__device__ __forceinline__ void twiddled_dft(Cx<Re>* v, int k, int ns, const Cx<Re>* tw) {
+  if (ns > 1) {
+    const Cx<Re>* q = tw + k + ns;
+#pragma unroll
+    for (int r = 1; r < R; ++r, q += ns) {
+      const Cx<Re> w = ldg(q);
+      v[r] = INV ? cmulc(v[r], w) : cmul(v[r], w);
+    }
+  }
+  Dft<R, INV, Re>::run(v);
+}
+
+// ---------------------------------------------------------------------------
+// runtime passes.  Each pass is a self-contained load -> twiddle -> butterfly
+// -> store under one radix dispatch, so its values live in registers only
+// inside the dispatched body.  (Keeping them across passes took two dispatches
+// per pass, butterflies and the next gather, with both layouts live.)
+// ---------------------------------------------------------------------------
+// Where a thread's transform lives in the exchange's shared memory: point i at
+// sm + i * pitch, padded by one slot every 16 points in rows of power-of-two
+// plans.  PADDED computes every slot (any radix list); otherwise the R points
+// of a butterfly, i0 + r di, are stepped through, one addition per access
+// instead of three operations.
+template <class Re, bool PADDED>
+struct Slots {
+  Cx<Re>* sm;  // slot of point 0
+  int pitch;   // slots between neighbouring points
+  int pad;     // 1 = padded rows (PassPlan::pad)
+  __device__ __forceinline__ Cx<Re>* at(int i) const {
+    return sm + (PADDED ? i + (i >> 4) : i * pitch + (i >> 4) * pad);
+  }
+  template <int R>
+  __device__ __forceinline__ void load(Cx<Re>* v, int i0, int di) const {
+    if constexpr (PADDED) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = *at(i0 + r * di);
+    } else {
+      const Cx<Re>* q = at(i0);
+      const int step = di * pitch + (di >> 4) * pad;
+#pragma unroll
+      for (int r = 0; r < R; ++r, q += step) v[r] = *q;
+    }
+  }
+  template <int R>
+  __device__ __forceinline__ void store(const Cx<Re>* v, int i0, int di) const {
+    if constexpr (PADDED) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) *at(i0 + r * di) = v[r];
+    } else {
+      Cx<Re>* q = at(i0);
+      const int step = di * pitch + (di >> 4) * pad;
+#pragma unroll
+      for (int r = 0; r < R; ++r, q += step) *q = v[r];
+    }
+  }
+};
+
+// The values of one pass.  They start as unspecified registers (no
+// instruction): left uninitialised, a body inside a loop keeps the values of
+// idle butterflies alive from one iteration to the next, for every radix of
+// the switch at once, and all of them spill (13 KB of spill stores in a
+// kernel of fifteen radices; 1500-point rows ran at 216 us).
+template <int N, class Re>
+struct Values {
+  Cx<Re> v[N];
+  __device__ __forceinline__ Values() {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      if constexpr (sizeof(Re) == 4) asm("" : "=f"(v[i].x), "=f"(v[i].y));
+      else asm("" : "=d"(v[i].x), "=d"(v[i].y));
+    }
+  }
+  __device__ __forceinline__ Cx<Re>* at(int i) { return v + i; }
+};
+
+// one pass of a plan: t = the thread's index in its transform, T = threads of
+// the transform, nb = butterflies, ns = product of the radices before it,
+// nsm = inv_magic(ns)
+struct PassAt {
+  int t, T, nb, ns;
+  unsigned nsm;
+  bool warp;  // the exchange stays inside a warp
+  __device__ __forceinline__ int k(int j) const { return ns > 1 ? mod_inv(j, ns, nsm) : 0; }
+};
+
+// source -> exchange (the plan's first pass, ns = 1).  smin: the source is the
+// exchange's own shared memory, so a barrier lies between.
+template <int R, int MAXE, bool INV, class Re, bool PADDED, class In>
+__device__ __forceinline__ void pass_head(PassAt a, Slots<Re, PADDED> x, const In& in, bool smin) {
+  Values<MAXE, Re> w;
+  Cx<Re>* v = w.v;
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { in.template load<R>(&v[b * R], j, a.nb); });
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { Dft<R, INV, Re>::run(&v[b * R]); });
+  if (smin) xsync(a.warp);
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { x.template store<R>(&v[b * R], j * R, 1); });
+  xsync(a.warp);
+}
+
+// exchange -> exchange
+template <int R, int MAXE, bool INV, class Re, bool PADDED>
+__device__ __forceinline__ void pass_mid(PassAt a, Slots<Re, PADDED> x, const Cx<Re>* tw) {
+  Values<MAXE, Re> w;
+  Cx<Re>* v = w.v;
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { x.template load<R>(&v[b * R], j, a.nb); });
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { twiddled_dft<R, INV>(&v[b * R], a.k(j), a.ns, tw); });
+  xsync(a.warp);
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) {
+    const int k = a.k(j);
+    x.template store<R>(&v[b * R], (j - k) * R + k, a.ns);
+  });
+  xsync(a.warp);
+}
+
+// exchange -> sink (the plan's last pass).  smout: the sink is the exchange's
+// own shared memory.
+template <int R, int MAXE, bool INV, class Re, bool PADDED, class Out>
+__device__ __forceinline__ void pass_tail(PassAt a, Slots<Re, PADDED> x, const Cx<Re>* tw, const Out& out,
+                                          bool smout) {
+  Values<MAXE, Re> w;
+  Cx<Re>* v = w.v;
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { x.template load<R>(&v[b * R], j, a.nb); });
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { twiddled_dft<R, INV>(&v[b * R], a.k(j), a.ns, tw); });
+  if (smout) xsync(a.warp);
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { out.template store<R>(&v[b * R], j, a.nb); });
+}
+
+// source -> sink (a plan of one pass: one thread holds a whole transform)
+template <int R, int MAXE, bool INV, class Re, class In, class Out>
+__device__ __forceinline__ void pass_only(PassAt a, const In& in, const Out& out) {
+  Values<MAXE, Re> w;
+  Cx<Re>* v = w.v;
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) {
+    in.template load<R>(&v[b * R], j, a.nb);
+    Dft<R, INV, Re>::run(&v[b * R]);
+    out.template store<R>(&v[b * R], j, a.nb);
+  });
+}
+
+// exchange -> last forward pass, spectrum operation, first inverse pass ->
+// exchange: both passes have the same radix and the same points
+template <int R, int MAXE, class Re, bool PADDED, class Op>
+__device__ __forceinline__ void pass_turn(PassAt a, Slots<Re, PADDED> x, const Cx<Re>* tw, const Op& op) {
+  Values<MAXE, Re> w;
+  Cx<Re>* v = w.v;
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { x.template load<R>(&v[b * R], j, a.nb); });
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) {
+    twiddled_dft<R, false>(&v[b * R], j, a.ns, tw);  // ns = nb in the last pass: k = j
+    op.template apply<R>(&v[b * R], j, a.nb);
+    Dft<R, true, Re>::run(&v[b * R]);
+  });
+  xsync(a.warp);
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { x.template store<R>(&v[b * R], j * R, 1); });
+  xsync(a.warp);
+}
+template <int R, int MAXE, class Re, class In, class Op, class Out>
+__device__ __forceinline__ void pass_turn_only(PassAt a, const In& in, const Op& op, const Out& out) {
+  Values<MAXE, Re> w;
+  Cx<Re>* v = w.v;
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) {
+    in.template load<R>(&v[b * R], j, a.nb);
+    Dft<R, false, Re>::run(&v[b * R]);
+    op.template apply<R>(&v[b * R], j, a.nb);
+    Dft<R, true, Re>::run(&v[b * R]);
+    out.template store<R>(&v[b * R], j, a.nb);
+  });
+}
+
+template <bool REV>
+__device__ __forceinline__ PassAt pass_at(const PassPlan& pp, int q, int ns, int t, bool warp) {
+  return PassAt{t, pp.T, pp.nb[REV ? pp.npass - 1 - q : q], ns, REV ? pp.nsmr[q] : pp.nsm[q], warp};
+}
+
+// passes 1 .. npass-2 (exchange to exchange) of a plan whose pass 0 ran radix
+// ns; returns the product of the radices run so far
+template <int MAXE, bool INV, bool REV, class Re, bool PADDED>
+__device__ __forceinline__ int middle_passes(const PassPlan& pp, int ns, int t, const Slots<Re, PADDED>& x,
+                                             const Cx<Re>* tw, bool warp) {
+  const int P = pp.npass;
+  for (int q = 1; q + 1 < P; ++q) {
+    const int R = pp.radix[REV ? P - 1 - q : q];
+    radix_dispatch(R, [&](auto rc) {
+      pass_mid<decltype(rc)::value, MAXE, INV>(pass_at<REV>(pp, q, ns, t, warp), x, tw);
+    });
+    ns *= R;
+  }
+  return ns;
+}
+
+// A whole transform of a runtime plan from source `in` to sink `out`.  smin /
+// smout: they live in the exchange's shared memory.
+template <int MAXE, bool INV, class Re, bool PADDED, class In, class Out>
+__device__ __forceinline__ void runtime_transform(const PassPlan& pp, int t, const Slots<Re, PADDED>& x,
+                                                  const Cx<Re>* tw, const In& in, const Out& out, bool smin,
+                                                  bool smout, bool warp) {
+  const int P = pp.npass, R0 = pp.radix[0];
+  if (P == 1) {
+    radix_dispatch(R0, [&](auto rc) {
+      pass_only<decltype(rc)::value, MAXE, INV, Re>(pass_at<false>(pp, 0, 1, t, warp), in, out);
+    });
+    return;
+  }
+  radix_dispatch(R0, [&](auto rc) {
+    pass_head<decltype(rc)::value, MAXE, INV>(pass_at<false>(pp, 0, 1, t, warp), x, in, smin);
+  });
+  const int ns = middle_passes<MAXE, INV, false>(pp, R0, t, x, tw, warp);
+  radix_dispatch(pp.radix[P - 1], [&](auto rc) {
+    pass_tail<decltype(rc)::value, MAXE, INV>(pass_at<false>(pp, P - 1, ns, t, warp), x, tw, out, smout);
+  });
+}
+
+// Forward transform, spectrum operation, inverse transform with the passes
+// reversed.
+template <int MAXE, class Re, bool PADDED, class In, class Op, class Out>
+__device__ __forceinline__ void runtime_convolve(const PassPlan& pp, int t, const Slots<Re, PADDED>& x,
+                                                 const Cx<Re>* tw, const Cx<Re>* twr, const In& in, const Op& op,
+                                                 const Out& out, bool warp) {
+  const int P = pp.npass, R0 = pp.radix[0], RL = pp.radix[P - 1];
+  if (P == 1) {
+    radix_dispatch(R0, [&](auto rc) {
+      pass_turn_only<decltype(rc)::value, MAXE, Re>(pass_at<false>(pp, 0, 1, t, warp), in, op, out);
+    });
+    return;
+  }
+  radix_dispatch(R0, [&](auto rc) {
+    pass_head<decltype(rc)::value, MAXE, false>(pass_at<false>(pp, 0, 1, t, warp), x, in, false);
+  });
+  int ns = middle_passes<MAXE, false, false>(pp, R0, t, x, tw, warp);
+  radix_dispatch(RL, [&](auto rc) {
+    pass_turn<decltype(rc)::value, MAXE>(pass_at<false>(pp, P - 1, ns, t, warp), x, tw, op);
+  });
+  ns = middle_passes<MAXE, true, true>(pp, RL, t, x, twr, warp);
+  radix_dispatch(R0, [&](auto rc) {
+    pass_tail<decltype(rc)::value, MAXE, true>(pass_at<true>(pp, P - 1, ns, t, warp), x, twr, out, false);
+  });
+}
+
+// ---------------------------------------------------------------------------
 // plan policies: how the kernels below learn n, T and the radix passes.
 //   DynPlan   - runtime pass list (any 13-smooth length), radix by switch
 //   FixPlan   - compile-time length, threads per transform and radix list;
@@ -335,9 +806,10 @@ struct RRev<RList<>, RList<Os...>> {
   using type = RList<Os...>;
 };
 
-template <int MAXE_>
+template <int MAXE_, bool PAD_ = true>
 struct DynPlan {
   static constexpr int MAXE = MAXE_;
+  static constexpr bool PAD = PAD_;
   __device__ __forceinline__ void assume_t(int) const {}
   const PassPlan& pp;
   __device__ __forceinline__ explicit DynPlan(const PassPlan& p) : pp(p) {}
@@ -356,31 +828,56 @@ struct DynPlan {
   __device__ __forceinline__ void run(Cx<Re>* v, const PL& pl, Cx<Re>* sm, const Cx<Re>* tw) const {
     run_passes<MAXE, INV>(v, pp, REV, pl, sm, tw, WarpLocal<PL>::value && warp_sized(pp.T));
   }
+  template <class Re, class PL>
+  __device__ __forceinline__ Slots<Re, !PL::kLinear> slots(const PL& pl, Cx<Re>* sm) const {
+    return Slots<Re, !PL::kLinear>{sm + pl.sidx(pp, 0), pl.pitch(pp), pl.pad(pp)};
+  }
+  // whole transform from source `in` to sink `out`; SMIN / SMOUT: in the
+  // exchange's shared memory
+  template <bool INV, bool SMIN, bool SMOUT, class PL, class Re, class In, class Out>
+  __device__ __forceinline__ void transform(const PL& pl, Cx<Re>* sm, const Cx<Re>* tw, const In& in,
+                                            const Out& out) const {
+    runtime_transform<MAXE, INV>(pp, pl.t, slots<Re>(pl, sm), tw, in, out, SMIN, SMOUT,
+                                 WarpLocal<PL>::value && warp_sized(pp.T));
+  }
+  template <class PL, class Re, class In, class Op, class Out>
+  __device__ __forceinline__ void convolve(const PL& pl, Cx<Re>* sm, const Cx<Re>* tw, const Cx<Re>* twr,
+                                           const In& in, const Op& op, const Out& out) const {
+    runtime_convolve<MAXE>(pp, pl.t, slots<Re>(pl, sm), tw, twr, in, op, out,
+                           WarpLocal<PL>::value && warp_sized(pp.T));
+  }
 };
 
-template <int N, int T, int MAXE, bool INV, class Re, class PL, int NS, int R, int... Rest>
+// FRESH: nothing in the exchange's shared memory is still being read, so the
+// first scatter needs no barrier before it
+template <int N, int T, int MAXE, bool INV, bool FRESH, class Re, class PL, int NS, int R, int... Rest>
 __device__ __forceinline__ void chain(Cx<Re>* v, const PassPlan& pp, const PL& pl, Cx<Re>* sm, const Cx<Re>* tw) {
   constexpr bool W = WarpLocal<PL>::value && warp_sized(T);
   butterflies<R, MAXE, INV, Re>(v, N / R, T, pl.t, NS, tw);
   if constexpr (sizeof...(Rest) > 0) {
-    xsync<W>();
-    scatter<R, MAXE, Re>(v, N / R, T, pl.t, NS, [&](int pos, Cx<Re> val) { sm[pl.sidx(pp, pos)] = val; });
+    if constexpr (!FRESH) xsync<W>();
+    each_butterfly<R, MAXE>(N / R, T, pl.t, [&](auto b, int j) {
+      const int k = j % NS;
+      xstore<R>(&v[b * R], sm, pp, pl, (j - k) * R + k, NS);
+    });
     xsync<W>();
     constexpr int R2 = RFirst<RList<Rest...>>::value;
-    gather<R2, MAXE, Re>(v, N / R2, T, pl.t, [&](int pos) { return sm[pl.sidx(pp, pos)]; });
-    chain<N, T, MAXE, INV, Re, PL, NS * R, Rest...>(v, pp, pl, sm, tw);
+    each_butterfly<R2, MAXE>(N / R2, T, pl.t, [&](auto b, int j) { xload<R2>(&v[b * R2], sm, pp, pl, j, N / R2); });
+    chain<N, T, MAXE, INV, false, Re, PL, NS * R, Rest...>(v, pp, pl, sm, tw);
   }
 }
 
-template <int N, int T, int MAXE, bool INV, class Re, class PL, int... Rs>
+template <int N, int T, int MAXE, bool INV, bool FRESH, class Re, class PL, int... Rs>
 __device__ __forceinline__ void chain_list(RList<Rs...>, Cx<Re>* v, const PassPlan& pp, const PL& pl, Cx<Re>* sm,
                                            const Cx<Re>* tw) {
-  chain<N, T, MAXE, INV, Re, PL, 1, Rs...>(v, pp, pl, sm, tw);
+  chain<N, T, MAXE, INV, FRESH, Re, PL, 1, Rs...>(v, pp, pl, sm, tw);
 }
 
 template <int N_, int T_, class L, int MAXE_ = 16>
 struct FixPlan {
   static constexpr int MAXE = MAXE_;
+  static constexpr bool PAD = true;
+  static constexpr int kFirst = RFirst<L>::value, kLast = RLast<L>::value;
   // the thread's index inside its transform is below T (lets the compiler
   // drop the j < n/R guards of exact plans)
   __device__ __forceinline__ void assume_t(int t) const { __builtin_assume(t >= 0 && t < T_); }
@@ -397,10 +894,34 @@ struct FixPlan {
     f(IC<REV ? RFirst<L>::value : RLast<L>::value>{});
   }
   // PL: a thread placement (Place<STRIDED> or any type with t and sidx(pp, i))
-  template <bool INV, bool REV, class PL, class Re>
+  template <bool INV, bool REV, bool FRESH = false, class PL, class Re>
   __device__ __forceinline__ void run(Cx<Re>* v, const PL& pl, Cx<Re>* sm, const Cx<Re>* tw) const {
     using Order = typename Cond<REV, typename RRev<L>::type, L>::type;
-    chain_list<N_, T_, MAXE, INV, Re, PL>(Order{}, v, pp, pl, sm, tw);
+    chain_list<N_, T_, MAXE, INV, FRESH, Re, PL>(Order{}, v, pp, pl, sm, tw);
+  }
+  // f(b, j) over the thread's butterflies of radix R
+  template <int R, class F>
+  __device__ __forceinline__ static void each(int t, F&& f) {
+    each_butterfly<R, MAXE>(N_ / R, T_, t, f);
+  }
+  template <bool INV, bool SMIN, bool SMOUT, class PL, class Re, class In, class Out>
+  __device__ __forceinline__ void transform(const PL& pl, Cx<Re>* sm, const Cx<Re>* tw, const In& in,
+                                            const Out& out) const {
+    Cx<Re> v[MAXE];
+    each<kFirst>(pl.t, [&](auto b, int j) { in.template load<kFirst>(&v[b * kFirst], j, N_ / kFirst); });
+    run<INV, false, !SMIN>(v, pl, sm, tw);
+    if constexpr (SMOUT) xsync<WarpLocal<PL>::value && warp_sized(T_)>();
+    each<kLast>(pl.t, [&](auto b, int j) { out.template store<kLast>(&v[b * kLast], j, N_ / kLast); });
+  }
+  template <class PL, class Re, class In, class Op, class Out>
+  __device__ __forceinline__ void convolve(const PL& pl, Cx<Re>* sm, const Cx<Re>* tw, const Cx<Re>* twr,
+                                           const In& in, const Op& op, const Out& out) const {
+    Cx<Re> v[MAXE];
+    each<kFirst>(pl.t, [&](auto b, int j) { in.template load<kFirst>(&v[b * kFirst], j, N_ / kFirst); });
+    run<false, false, true>(v, pl, sm, tw);
+    each<kLast>(pl.t, [&](auto b, int j) { op.template apply<kLast>(&v[b * kLast], j, N_ / kLast); });
+    run<true, true>(v, pl, sm, twr);
+    each<kFirst>(pl.t, [&](auto b, int j) { out.template store<kFirst>(&v[b * kFirst], j, N_ / kFirst); });
   }
 };
 
@@ -427,46 +948,27 @@ __device__ __forceinline__ Cx<Re>* smem_base() {
   return reinterpret_cast<Cx<Re>*>(vdx_smem_raw);
 }
 
-// First-pass gather of a complex input (signal-range masked).  CTAs whose
-// slots all exist and whose range is the whole axis take the unpredicated
-// path.
-template <class Plan, class S, class Re, bool STRIDED>
-__device__ __forceinline__ void gather_input(const Plan& P, const Place<STRIDED>& pl, const FftArgs& a, Cx<Re>* v,
-                                             const S* in) {
-  constexpr int MAXE = Plan::MAXE;
-  const int n = P.n();
-  const int lo = a.sig_lo, hi = a.sig_hi;
-  if (pl.tile_full && lo <= 0 && hi >= n) {
-    P.template first<false>([&](auto rc) {
-      constexpr int RR = decltype(rc)::value;
-      gather<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos) { return Conv<S, Re>::ld(in + pos * pl.ps); });
-    });
-  } else {
-    P.template first<false>([&](auto rc) {
-      constexpr int RR = decltype(rc)::value;
-      gather<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos) {
-        if (!pl.valid || pos < lo || pos >= hi) return mk<Re>(Re(0), Re(0));
-        return Conv<S, Re>::ld(in + pos * pl.ps);
-      });
-    });
-  }
+// First-pass gather and last-pass store of kernels that keep a transform's
+// values in registers across the passes.
+template <class Plan, class S, class Re, bool STRIDED, bool PAD>
+__device__ __forceinline__ void gather_input(const Plan& P, const Place<STRIDED, PAD>& pl, const FftArgs& a,
+                                             Cx<Re>* v) {
+  const GlobalIn<S, Re> in(a, pl, P.n());
+  P.template first<false>([&](auto rc) {
+    constexpr int RR = decltype(rc)::value;
+    const int nb = P.n() / RR;
+    each_butterfly<RR, Plan::MAXE>(nb, P.T(), pl.t, [&](auto b, int j) { in.template load<RR>(&v[b * RR], j, nb); });
+  });
 }
 
-// Natural-order store of the last executed pass, scaled, to `base` (a.out
-// unless given) at the thread's transform offset.
-template <class Plan, bool REV, class S, class Re, bool STRIDED>
-__device__ __forceinline__ void store_output(const Plan& P, const Place<STRIDED>& pl, const FftArgs& a, Cx<Re>* v,
+template <class Plan, bool REV, class S, class Re, bool STRIDED, bool PAD>
+__device__ __forceinline__ void store_output(const Plan& P, const Place<STRIDED, PAD>& pl, const FftArgs& a, Cx<Re>* v,
                                              S* base = nullptr) {
-  constexpr int MAXE = Plan::MAXE;
-  S* out = (base ? base : reinterpret_cast<S*>(a.out)) + pl.out0();
-  const int n = P.n();
-  const Re s = Re(a.scale);
-  const bool all = pl.tile_full;
+  const GlobalOut<S, Re> out(a, pl, base);
   P.template last<REV>([&](auto rc) {
     constexpr int RR = decltype(rc)::value;
-    each_natural<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos, Cx<Re> val) {
-      if (all || pl.valid) Conv<S, Re>::st(out + pos * pl.ps, scale(val, s));
-    });
+    const int nb = P.n() / RR;
+    each_butterfly<RR, Plan::MAXE>(nb, P.T(), pl.t, [&](auto b, int j) { out.template store<RR>(&v[b * RR], j, nb); });
   });
 }
 
@@ -482,52 +984,15 @@ template <class Plan, bool INV, bool STRIDED, class S, class Re, int IW = 0, int
 __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 32 ? 2 : 1) k_c2c(FftArgs a) {
   pdl_enter();
   const Plan P(a.pp);
-  constexpr int MAXE = Plan::MAXE;
-  const Place<STRIDED> pl(a, P.T());
+  const Place<STRIDED, Plan::PAD> pl(a, P.T());
   Cx<Re>* sm = smem_base<Re>();
   const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
-  const S* in = reinterpret_cast<const S*>(a.in) + pl.in0();
-  Cx<Re> v[MAXE];
   P.assume_t(pl.t);
-  const int n = P.n();
-  gather_input<Plan, S, Re>(P, pl, a, v, in);
   if constexpr (IW) {
-    const float* w = a.in_weight + pl.in0();
-    const Re f = Re(a.in_weight_scale) * (a.in_weight_scale_ptr ? Re(__ldg(a.in_weight_scale_ptr)) : Re(1));
-    const bool ok = pl.tile_full || pl.valid;
-    P.template first<false>([&](auto rc) {
-      constexpr int RR = decltype(rc)::value;
-      constexpr int B = MAXE / RR;
-      const int nb = n / RR;
-#pragma unroll
-      for (int b = 0; b < B; ++b) {
-        const int j = pl.t + b * P.T();
-        if (j < nb) {
-#pragma unroll
-          for (int r = 0; r < RR; ++r) {
-            const Re wv = ok ? Re(__ldg(w + (j + r * nb) * pl.ps)) * f : Re(0);
-            v[b * RR + r] = scale(v[b * RR + r], wv);
-          }
-        }
-      }
-    });
-  }
-  P.template run<INV, false>(v, pl, sm, tw);
-  store_output<Plan, false, S, Re>(P, pl, a, v);
-  if constexpr (LOSS) {
-    const float* lw = a.loss_weight + pl.out0();
-    const Re s = Re(a.scale);
-    const bool ok = pl.tile_full || pl.valid;
+    P.template transform<INV, false, false>(pl, sm, tw, WeightedIn<S, Re>(a, pl, P.n()), GlobalOut<S, Re>(a, pl));
+  } else if constexpr (LOSS) {
     float acc = 0.f;
-    P.template last<false>([&](auto rc) {
-      constexpr int RR = decltype(rc)::value;
-      each_natural<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos, Cx<Re> val) {
-        if (ok) {
-          const Cx<Re> y = scale(val, s);
-          acc += __ldg(lw + pos * pl.ps) * float(y.x * y.x + y.y * y.y);
-        }
-      });
-    });
+    P.template transform<INV, false, false>(pl, sm, tw, GlobalIn<S, Re>(a, pl, P.n()), LossOut<S, Re>(a, pl, &acc));
     // block sum in a fixed order through shared memory (any CTA size; the
     // plan reserves blockDim floats of dynamic shared memory)
     float* red = reinterpret_cast<float*>(sm);
@@ -542,6 +1007,8 @@ __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 3
       __syncthreads();
     }
     if (tid == 0) a.loss_partials[blockIdx.x] = red[0];
+  } else {
+    P.template transform<INV, false, false>(pl, sm, tw, GlobalIn<S, Re>(a, pl, P.n()), GlobalOut<S, Re>(a, pl));
   }
 }
 
@@ -557,55 +1024,13 @@ template <class Plan, bool STRIDED, class S, class K, class Re, int KOP, int SPE
 __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 32 ? 2 : 1) k_conv(FftArgs a) {
   pdl_enter();
   const Plan P(a.pp);
-  constexpr int MAXE = Plan::MAXE;
-  const Place<STRIDED> pl(a, P.T());
+  const Place<STRIDED, Plan::PAD> pl(a, P.T());
   Cx<Re>* sm = smem_base<Re>();
   const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
   const Cx<Re>* twr = reinterpret_cast<const Cx<Re>*>(a.twr);
-  const S* in = reinterpret_cast<const S*>(a.in) + pl.in0();
-  Cx<Re> v[MAXE];
   P.assume_t(pl.t);
-  const int n = P.n();
-  gather_input<Plan, S, Re>(P, pl, a, v, in);
-  const bool kvalid = pl.tile_full || pl.valid;
-  P.template run<false, false>(v, pl, sm, tw);
-  if constexpr (SPEC != 0) {
-    S* so = reinterpret_cast<S*>(a.spec_out) + pl.out0();
-    const S* sa = reinterpret_cast<const S*>(a.spec_aux) + pl.out0();
-    const Re ss = Re(a.spec_scale);
-    P.template last<false>([&](auto rc) {
-      constexpr int RR = decltype(rc)::value;
-      each_natural<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos, Cx<Re> val) {
-        if (!kvalid) return;
-        if (SPEC == 1) {
-          Conv<S, Re>::st(so + pos * pl.ps, val);
-        } else {
-          const Cx<Re> x = Conv<S, Re>::ld(sa + pos * pl.ps);
-          Conv<S, Re>::st(so + pos * pl.ps, scale(cmulc(x, val), ss));
-        }
-      });
-    });
-  }
-  const K* ker = reinterpret_cast<const K*>(a.ker) + pl.ker0();
-  P.template last<false>([&](auto rc) {
-    constexpr int RR = decltype(rc)::value;
-    constexpr int B = MAXE / RR;
-    const int nb = n / RR;
-#pragma unroll
-    for (int b = 0; b < B; ++b) {
-      const int j = pl.t + b * P.T();
-      if (j < nb) {
-#pragma unroll
-        for (int r = 0; r < RR; ++r) {
-          const int pos = j + r * nb;
-          Cx<Re> kv = kvalid ? Conv<K, Re>::ld(ker + pos * pl.ps) : mk<Re>(Re(0), Re(0));
-          v[b * RR + r] = KOP == 0 ? cmulc(v[b * RR + r], kv) : cmul(v[b * RR + r], kv);
-        }
-      }
-    }
-  });
-  P.template run<true, true>(v, pl, sm, twr);
-  store_output<Plan, true, S, Re>(P, pl, a, v);
+  P.convolve(pl, sm, tw, twr, GlobalIn<S, Re>(a, pl, P.n()), SpectrumOp<S, K, Re, KOP, SPEC>(a, pl),
+             GlobalOut<S, Re>(a, pl));
 }
 
 // Strided fused convolution for CTAs of at most 256 threads, complex64.  The
@@ -624,14 +1049,13 @@ __global__ void __launch_bounds__(256, Plan::MAXE <= 8 ? 3 : 2) k_conv_pf(FftArg
   Cx<Re>* sm = smem_base<Re>();
   const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
   const Cx<Re>* twr = reinterpret_cast<const Cx<Re>*>(a.twr);
-  const S* in = reinterpret_cast<const S*>(a.in) + pl.in0();
   const S* ker = reinterpret_cast<const S*>(a.ker) + pl.ker0();
   P.assume_t(pl.t);
   const int n = P.n();
   const bool kvalid = pl.tile_full || pl.valid;
   constexpr bool PF = MAXE <= 16;
   Cx<Re> v[MAXE];
-  gather_input<Plan, S, Re>(P, pl, a, v, in);
+  gather_input<Plan, S, Re>(P, pl, a, v);
   Cx<Re> kr[PF ? MAXE : 1];
   if constexpr (PF) P.template last<false>([&](auto rc) {
     constexpr int RR = decltype(rc)::value;
@@ -640,29 +1064,31 @@ __global__ void __launch_bounds__(256, Plan::MAXE <= 8 ? 3 : 2) k_conv_pf(FftArg
 #pragma unroll
     for (int b = 0; b < B; ++b) {
       const int j = pl.t + b * P.T();
+      const S* q = ker + j * pl.ps;
+      const long long step = nb * pl.ps;
 #pragma unroll
-      for (int r = 0; r < RR; ++r)
-        kr[b * RR + r] = (j < nb && kvalid) ? ld_once<S, Re>(ker + (j + r * nb) * pl.ps) : mk<Re>(Re(0), Re(0));
+      for (int r = 0; r < RR; ++r, q += step)
+        kr[b * RR + r] = (j < nb && kvalid) ? ld_once<S, Re>(q) : mk<Re>(Re(0), Re(0));
     }
   });
-  P.template run<false, false>(v, pl, sm, tw);
+  P.template run<false, false, true>(v, pl, sm, tw);
   P.template last<false>([&](auto rc) {
     constexpr int RR = decltype(rc)::value;
     constexpr int B = MAXE / RR;
     const int nb = n / RR;
 #pragma unroll
-    for (int b = 0; b < B; ++b)
+    for (int b = 0; b < B; ++b) {
+      const int j = pl.t + b * P.T();
+      const S* q = ker + j * pl.ps;
+      const long long step = nb * pl.ps;
 #pragma unroll
-      for (int r = 0; r < RR; ++r) {
+      for (int r = 0; r < RR; ++r, q += step) {
         Cx<Re> k;
-        if constexpr (PF) {
-          k = kr[b * RR + r];
-        } else {
-          const int j = pl.t + b * P.T();
-          k = (j < nb && kvalid) ? ld_once<S, Re>(ker + (j + r * nb) * pl.ps) : mk<Re>(Re(0), Re(0));
-        }
+        if constexpr (PF) k = kr[b * RR + r];
+        else k = (j < nb && kvalid) ? ld_once<S, Re>(q) : mk<Re>(Re(0), Re(0));
         v[b * RR + r] = KOP == 0 ? cmulc(v[b * RR + r], k) : cmul(v[b * RR + r], k);
       }
+    }
   });
   P.template run<true, true>(v, pl, sm, twr);
   store_output<Plan, true, S, Re>(P, pl, a, v);
@@ -682,18 +1108,17 @@ __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 3
   pdl_enter();
   const Plan P(a.pp);
   constexpr int MAXE = Plan::MAXE;
-  const Place<STRIDED> pl(a, P.T());
+  const Place<STRIDED, Plan::PAD> pl(a, P.T());
   Cx<Re>* sm = smem_base<Re>();
   const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
   const Cx<Re>* twr = reinterpret_cast<const Cx<Re>*>(a.twr);
   unsigned dyn;
   asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
   Cx<Re>* keep = sm + (dyn / sizeof(Cx<Re>) - unsigned(MAXE) * blockDim.x);
-  const S* in = reinterpret_cast<const S*>(a.in) + pl.in0();
   Cx<Re> v[MAXE];
   P.assume_t(pl.t);
   const int n = P.n();
-  gather_input<Plan, S, Re>(P, pl, a, v, in);
+  gather_input<Plan, S, Re>(P, pl, a, v);
   const bool kvalid = pl.tile_full || pl.valid;
   P.template run<false, false>(v, pl, sm, tw);
 #pragma unroll
@@ -729,127 +1154,124 @@ __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 3
 // ---------------------------------------------------------------------------
 // real-to-complex, even N = 2n, rows of the packed RFFT layout: row pitch
 // n+1 complex elements = 2n+2 reals (vkdispatch/base/buffer.py:377-448).
-// z[m] = x[2m] + i x[2m+1] -> Z = FFT_n(z) ->
-// X[k] = (Z[k] + conj Z[n-k])/2 - i W_2n^k (Z[k] - conj Z[n-k])/2, k = 0..n
+// z[m] = x[2m] + i x[2m+1] -> Z = FFT_n(z) -> with e = (Z[k] + conj Z[n-k])/2
+// and o = (Z[k] - conj Z[n-k])/2i:
+//   X[k] = e + W_2n^k o,   X[n-k] = conj(e - W_2n^k o),   k = 0..n/2
+// One thread forms both bins of a pair, so a pair costs one twiddle product
+// and two shared-memory reads.
 // ---------------------------------------------------------------------------
+// packed real row as complex points; the signal range counts reals
+template <class S, class Re>
+struct RealIn {
+  const S* p;
+  int lo, hi;
+  bool full, valid;
+  template <class PL>
+  __device__ __forceinline__ RealIn(const FftArgs& a, const PL& pl, int n)
+      : p(reinterpret_cast<const S*>(a.in) + pl.in0()), lo(a.sig_lo), hi(a.sig_hi),
+        full(a.sig_lo <= 0 && a.sig_hi >= 2 * n && pl.tile_full), valid(pl.valid) {}
+  template <int R>
+  __device__ __forceinline__ void load(Cx<Re>* v, int j, int nb) const {
+    using SR = typename RealOf<S>::type;
+    if (full) {
+      const S* q = p + j;
+#pragma unroll
+      for (int r = 0; r < R; ++r, q += nb) v[r] = Conv<S, Re>::ld(q);
+      return;
+    }
+    const SR* pr = reinterpret_cast<const SR*>(p);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int e = 2 * (j + r * nb), o = e + 1;
+      const Re xr = valid && e >= lo && e < hi ? ld_real<Re>(pr + e) : Re(0);
+      const Re xi = valid && o >= lo && o < hi ? ld_real<Re>(pr + o) : Re(0);
+      v[r] = mk<Re>(xr, xi);
+    }
+  }
+};
+
 template <class Plan, class S, class Re>
 __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 32 ? 2 : 1) k_r2c_even(FftArgs a) {
   pdl_enter();
-  using SR = typename RealOf<S>::type;
   const Plan P(a.pp);
-  constexpr int MAXE = Plan::MAXE;
-  const Place<false> pl(a, P.T());
-  const PassPlan& pp = a.pp;
+  const Place<false, Plan::PAD> pl(a, P.T());
   Cx<Re>* sm = smem_base<Re>();
   const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
   const Cx<Re>* tw2 = reinterpret_cast<const Cx<Re>*>(a.tw2);
-  const S* in = reinterpret_cast<const S*>(a.in) + pl.in0();
-  const SR* inr = reinterpret_cast<const SR*>(in);
-  S* out = reinterpret_cast<S*>(a.out) + pl.out0();
-  Cx<Re> v[MAXE];
   P.assume_t(pl.t);
   const int n = P.n();
-  const int lo = a.sig_lo, hi = a.sig_hi;
-  const bool full = lo <= 0 && hi >= 2 * n && pl.tile_full;
-  P.template first<false>([&](auto rc) {
-    constexpr int RR = decltype(rc)::value;
-    if (full) {
-      gather<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos) { return Conv<S, Re>::ld(in + pos); });
-      return;
-    }
-    gather<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos) {
-      if (!pl.valid) return mk<Re>(Re(0), Re(0));
-      const int e = 2 * pos, o = 2 * pos + 1;
-      Re xr = (e >= lo && e < hi) ? ld_real<Re>(inr + e) : Re(0);
-      Re xi = (o >= lo && o < hi) ? ld_real<Re>(inr + o) : Re(0);
-      return mk<Re>(xr, xi);
-    });
-  });
-  P.template run<false, false>(v, pl, sm, tw);
-  const bool wsync = warp_sized(P.T());  // rows: the exchange below stays inside the row's warp
-  xsync(wsync);
-  P.template last<false>([&](auto rc) {
-    constexpr int RR = decltype(rc)::value;
-    each_natural<RR, MAXE, Re>(v, n / RR, P.T(), pl.t,
-                               [&](int pos, Cx<Re> val) { sm[pl.sidx_plain(pp, pos)] = val; });
-  });
-  xsync(wsync);
+  Cx<Re>* z = sm + pl.sidx_plain(a.pp, 0);
+  P.template transform<false, false, true>(pl, sm, tw, RealIn<S, Re>(a, pl, n), SharedOut<Re>{z});
+  xsync(warp_sized(P.T()));  // rows: the exchange stays inside the row's warp
+  if (!(pl.tile_full || pl.valid)) return;
+  S* out = reinterpret_cast<S*>(a.out) + pl.out0();
   const Re half = Re(0.5);
-  const bool wr = pl.tile_full || pl.valid;
-  P.template last<false>([&](auto rc) {
-    constexpr int RR = decltype(rc)::value;
-    each_natural<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int k, Cx<Re> zk) {
-      const int kc = k == 0 ? 0 : n - k;
-      const Cx<Re> zc = conj(sm[pl.sidx_plain(pp, kc)]);
-      const Cx<Re> e = scale(zk + zc, half);
-      const Cx<Re> d = scale(zk - zc, half);
-      const Cx<Re> o = mk<Re>(d.y, -d.x);  // d / i
-      const Cx<Re> x = e + cmul(ldg(&tw2[k]), o);
-      if (wr) Conv<S, Re>::st(out + k, x);
-    });
-  });
-  if (pl.t == 0 && pl.valid) {
-    const Cx<Re> z0 = sm[pl.sidx_plain(pp, 0)];
-    Conv<S, Re>::st(out + n, mk<Re>(z0.x - z0.y, Re(0)));
+  // n <= T * MAXE for every plan, so MAXE/2 steps cover every pair
+#pragma unroll
+  for (int u = 0; u <= Plan::MAXE / 2; ++u) {
+    const int k = pl.t + u * P.T();
+    if (2 * k > n) break;
+    const Cx<Re> zk = z[k], zc = conj(z[k == 0 ? 0 : n - k]);
+    const Cx<Re> e = scale(zk + zc, half);
+    const Cx<Re> d = scale(zk - zc, half);
+    const Cx<Re> wo = cmul(ldg(&tw2[k]), mk<Re>(d.y, -d.x));  // d / i
+    Conv<S, Re>::st(out + k, e + wo);
+    if (k == 0) Conv<S, Re>::st(out + n, mk<Re>(zk.x - zk.y, Re(0)));
+    else if (2 * k != n) Conv<S, Re>::st(out + (n - k), conj(e - wo));
   }
 }
 
 // ---------------------------------------------------------------------------
-// complex-to-real, even N = 2n (Hermitian half X[0..n] -> N reals).
-// Z[k] = (X[k] + conj X[n-k]) + i W_2n^{-k} (X[k] - conj X[n-k]), with the
-// imaginary parts of X[0] and X[n] dropped (the real part of the full-length
-// inverse does not depend on them) -> z = IFFT_n(Z) -> x[2m] + i x[2m+1] = z[m]
+// complex-to-real, even N = 2n (Hermitian half X[0..n] -> N reals).  With
+// s = X[k] + conj X[n-k] and w = W_2n^{-k} (X[k] - conj X[n-k]):
+//   Z[k] = s + i w,   Z[n-k] = conj(s - i w),   k = 0..n/2,
+// with the imaginary parts of X[0] and X[n] dropped (the real part of the
+// full-length inverse does not depend on them) -> z = IFFT_n(Z) ->
+// x[2m] + i x[2m+1] = z[m]
 // ---------------------------------------------------------------------------
 template <class Plan, class S, class Re>
 __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 32 ? 2 : 1) k_c2r_even(FftArgs a) {
   pdl_enter();
   const Plan P(a.pp);
-  constexpr int MAXE = Plan::MAXE;
-  const Place<false> pl(a, P.T());
-  const PassPlan& pp = a.pp;
+  const Place<false, Plan::PAD> pl(a, P.T());
   Cx<Re>* sm = smem_base<Re>();
   const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
   const Cx<Re>* tw2 = reinterpret_cast<const Cx<Re>*>(a.tw2);
   const S* in = reinterpret_cast<const S*>(a.in) + pl.in0();
-  Cx<Re> v[MAXE];
   P.assume_t(pl.t);
   const int n = P.n();
-  // X[0..n-1] through registers with every load in flight before the first
-  // shared-memory store (n <= T * MAXE for every plan); X[n] by thread 0
-  const bool ld_ok = pl.tile_full || pl.valid;
+  Cx<Re>* z = sm + pl.sidx_plain(a.pp, 0);
+  if (pl.tile_full || pl.valid) {
+    constexpr int U = Plan::MAXE / 2;  // pairs per thread (n <= T * MAXE), the middle bin apart
+    Cx<Re> lo[U], hi[U];
+    // every load in flight before the first shared-memory store
 #pragma unroll
-  for (int u = 0; u < MAXE; ++u) {
-    const int i = pl.t + u * P.T();
-    if (i < n) v[u] = ld_ok ? Conv<S, Re>::ld(in + i) : mk<Re>(Re(0), Re(0));
-  }
+    for (int u = 0; u < U; ++u) {
+      const int k = pl.t + u * P.T();
+      if (2 * k < n) {
+        lo[u] = Conv<S, Re>::ld(in + k);
+        hi[u] = Conv<S, Re>::ld(in + (n - k));
+      }
+    }
+    if (n % 2 == 0 && pl.t == 0) {
+      const Cx<Re> x = Conv<S, Re>::ld(in + n / 2);
+      z[n / 2] = mk<Re>(x.x + x.x, -(x.y + x.y));  // s = 2 Re x, w = -2 Im x
+    }
 #pragma unroll
-  for (int u = 0; u < MAXE; ++u) {
-    const int i = pl.t + u * P.T();
-    if (i < n) {
-      Cx<Re> x = v[u];
-      if (i == 0) x.y = Re(0);
-      sm[pl.sidx_plain(pp, i)] = x;
+    for (int u = 0; u < U; ++u) {
+      const int k = pl.t + u * P.T();
+      if (2 * k < n) {
+        Cx<Re> xk = lo[u], xc = conj(hi[u]);
+        if (k == 0) xk.y = xc.y = Re(0);
+        const Cx<Re> s = xk + xc;
+        const Cx<Re> w = cmulc(xk - xc, ldg(&tw2[k]));  // * W^{-k}
+        z[k] = mk<Re>(s.x - w.y, s.y + w.x);
+        if (k != 0) z[n - k] = mk<Re>(s.x + w.y, w.x - s.y);
+      }
     }
   }
-  if (pl.t == 0) {
-    Cx<Re> x = ld_ok ? Conv<S, Re>::ld(in + n) : mk<Re>(Re(0), Re(0));
-    x.y = Re(0);
-    sm[pl.sidx_plain(pp, n)] = x;
-  }
   xsync(warp_sized(P.T()));  // rows: the exchange stays inside the row's warp
-  P.template first<false>([&](auto rc) {
-    constexpr int RR = decltype(rc)::value;
-    gather<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int k) {
-      const Cx<Re> xk = sm[pl.sidx_plain(pp, k)];
-      const Cx<Re> xc = conj(sm[pl.sidx_plain(pp, n - k)]);
-      const Cx<Re> s = xk + xc;
-      const Cx<Re> d = xk - xc;
-      const Cx<Re> wd = cmulc(d, ldg(&tw2[k]));  // d * W^{-k}
-      return mk<Re>(s.x - wd.y, s.y + wd.x);     // s + i*wd
-    });
-  });
-  P.template run<true, false>(v, pl, sm, tw);
-  store_output<Plan, false, S, Re>(P, pl, a, v);
+  P.template transform<true, true, false>(pl, sm, tw, SharedIn<Re>{z}, GlobalOut<S, Re>(a, pl));
 }
 
 // ---------------------------------------------------------------------------
@@ -859,46 +1281,57 @@ __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 3
 // reference's own R2C I/O rules (vkdispatch/fft/global_memory_iterators.py:
 // 85-92, 214-226).  Row pitch N+1 reals = N/2+1 complex.
 // ---------------------------------------------------------------------------
+template <bool INV, class S, class Re>
+struct OddIn {
+  const S* p;
+  int n, lo, hi;
+  bool valid;
+  template <int R>
+  __device__ __forceinline__ void load(Cx<Re>* v, int j, int nb) const {
+    using SR = typename RealOf<S>::type;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int pos = j + r * nb;
+      if (!valid) v[r] = mk<Re>(Re(0), Re(0));
+      else if (!INV)
+        v[r] = mk<Re>(pos >= lo && pos < hi ? ld_real<Re>(reinterpret_cast<const SR*>(p) + pos) : Re(0), Re(0));
+      else v[r] = pos <= n / 2 ? Conv<S, Re>::ld(p + pos) : conj(Conv<S, Re>::ld(p + (n - pos)));
+    }
+  }
+};
+template <bool INV, class S, class Re>
+struct OddOut {
+  S* p;
+  int n;
+  Re s;
+  bool valid;
+  template <int R>
+  __device__ __forceinline__ void store(const Cx<Re>* v, int j, int nb) const {
+    using SR = typename RealOf<S>::type;
+    if (!valid) return;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int pos = j + r * nb;
+      if (INV) st_real<Re>(reinterpret_cast<SR*>(p) + pos, v[r].x * s);
+      else if (pos <= n / 2) Conv<S, Re>::st(p + pos, v[r]);
+    }
+  }
+};
+
+// In place, every row is read whole before its first store only because the
+// passes exchange through shared memory; a one-pass transform stores after
+// its own loads, and one thread holds the whole row.
 template <class Plan, bool INV, class S, class Re>
 __global__ void __launch_bounds__(1024) k_real_odd(FftArgs a) {
   pdl_enter();
-  using SR = typename RealOf<S>::type;
   const Plan P(a.pp);
-  constexpr int MAXE = Plan::MAXE;
-  const Place<false> pl(a, P.T());
+  const Place<false, Plan::PAD> pl(a, P.T());
   Cx<Re>* sm = smem_base<Re>();
   const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
-  const S* in = reinterpret_cast<const S*>(a.in) + pl.in0();
-  S* out = reinterpret_cast<S*>(a.out) + pl.out0();
-  Cx<Re> v[MAXE];
   const int n = P.n();
-  const int h = n / 2;
-  const int lo = a.sig_lo, hi = a.sig_hi;
-  P.template first<false>([&](auto rc) {
-    constexpr int RR = decltype(rc)::value;
-    gather<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos) {
-      if (!pl.valid) return mk<Re>(Re(0), Re(0));
-      if (!INV) {
-        if (pos < lo || pos >= hi) return mk<Re>(Re(0), Re(0));
-        return mk<Re>(ld_real<Re>(reinterpret_cast<const SR*>(in) + pos), Re(0));
-      }
-      if (pos <= h) return Conv<S, Re>::ld(in + pos);
-      return conj(Conv<S, Re>::ld(in + (n - pos)));
-    });
-  });
-  P.template run<INV, false>(v, pl, sm, tw);
-  const Re s = Re(a.scale);
-  P.template last<false>([&](auto rc) {
-    constexpr int RR = decltype(rc)::value;
-    each_natural<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos, Cx<Re> val) {
-      if (!pl.valid) return;
-      if (!INV) {
-        if (pos <= h) Conv<S, Re>::st(out + pos, val);
-      } else {
-        st_real<Re>(reinterpret_cast<SR*>(out) + pos, val.x * s);
-      }
-    });
-  });
+  P.template transform<INV, false, false>(
+      pl, sm, tw, OddIn<INV, S, Re>{reinterpret_cast<const S*>(a.in) + pl.in0(), n, a.sig_lo, a.sig_hi, pl.valid},
+      OddOut<INV, S, Re>{reinterpret_cast<S*>(a.out) + pl.out0(), n, Re(a.scale), pl.valid});
 }
 
 // ---------------------------------------------------------------------------

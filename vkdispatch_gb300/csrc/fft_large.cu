@@ -26,210 +26,11 @@
 #include <cstring>
 #include <mutex>
 
-#include "fft_kernels.cuh"
-#include "tc_ptx.cuh"
-#include "vdx_internal.h"
+#include "fft_large.cuh"
 
 namespace vdx {
 
 namespace {
-
-// thread placement inside a column tile: m = column, t = thread of the column
-// (the interface run_passes / FixPlan::run use)
-struct FsPlace {
-  int t, m, M;
-  __device__ __forceinline__ int sidx(const PassPlan&, int i) const { return i * M + m; }
-};
-
-// MODE 0: plain store (pass B).  MODE 1: four-step twiddle, then a store
-// whose columns are unit-stride (strided axes).  MODE 2: four-step twiddle,
-// then a transposed store through shared memory so that each column's points
-// land contiguously (out_ps == 1; contiguous axes).
-// TMA tile copies: dims (columns, then the other axes by increasing stride),
-// coordinates in that order; the box is M columns x n rows.
-struct TmaTile {
-  int rank;
-  int row_dim, br_dim, bq_dim;  // position of each in the map (-1: not a dimension)
-};
-constexpr long long kTmaWait = 1ll << 24;  // polls before a tile-load wait gives up
-
-template <int RANK>
-__device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap* map, const int* c, uint64_t* bar) {
-  const uint64_t m = reinterpret_cast<uint64_t>(map);
-  const uint32_t b = tc::smem_u32(bar);
-  if constexpr (RANK == 2) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            dst),
-        "l"(m), "r"(c[0]), "r"(c[1]), "r"(b)
-        : "memory");
-  } else if constexpr (RANK == 3) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            dst),
-        "l"(m), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(b)
-        : "memory");
-  } else {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-        "[%6];" ::"r"(dst),
-        "l"(m), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(b)
-        : "memory");
-  }
-}
-
-// TMA > 0: the input tile arrives by one bulk-tensor copy of rank TMA into
-// shared memory behind the exchange area, and the first pass gathers from it.
-template <class Plan, bool INV, class S, int MODE, int TMA>
-__global__ void __launch_bounds__(512) k_fs(const __grid_constant__ CUtensorMap tmap, FsArgs a, TmaTile tt) {
-  using Re = float;
-  const Plan P(a.pp);
-  constexpr int MAXE = Plan::MAXE;
-  const int M = a.pp.M;
-  FsPlace pl;
-  pl.M = M;
-  pl.m = threadIdx.x % M;
-  pl.t = threadIdx.x / M;
-  P.assume_t(pl.t);
-  const int n = P.n();
-  const int tile = blockIdx.x % a.col_tiles;
-  const long long b = blockIdx.x / a.col_tiles;
-  const long long bq = b / a.split, br = b - bq * a.split;
-  const int col = tile * M + pl.m;
-  const bool valid = col < a.ncols;
-  Cx<Re>* sm = smem_base<Re>();
-  const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
-  Cx<Re> v[MAXE];
-  if constexpr (TMA > 0) {
-    // staging after the exchange area ((n + 1) * M complex slots), on the
-    // 128-byte boundary a tensor copy's destination needs
-    const uint32_t stg_addr = (tc::smem_u32(sm + (n + 1) * M) + 127u) & ~127u;
-    const S* stg = reinterpret_cast<const S*>(reinterpret_cast<const unsigned char*>(sm) +
-                                              (stg_addr - tc::smem_u32(sm)));
-    __shared__ __align__(8) uint64_t bar;
-    if (threadIdx.x == 0) {
-      tc::mbar_init(&bar, 1);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const uint32_t bytes = uint32_t(n) * uint32_t(M) * uint32_t(sizeof(S));
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(&bar)), "r"(bytes)
-                   : "memory");
-      int c[4] = {0, 0, 0, 0};
-      c[0] = tile * M;
-      if (tt.br_dim >= 0) c[tt.br_dim] = (int)br;
-      if (tt.bq_dim >= 0) c[tt.bq_dim] = (int)bq;
-      tma_load<TMA>(stg_addr, &tmap, c, &bar);
-    }
-    if (!__syncthreads_and(tc::mbar_wait(&bar, 0, kTmaWait))) {
-      if (threadIdx.x == 0 && a.status) atomicExch(a.status, 1);
-      tc::mbar_wait(&bar, 0, kTmaWait);  // the copy is still in flight: let it land before leaving
-      return;
-    }
-    P.template first<false>([&](auto rc) {
-      constexpr int RR = decltype(rc)::value;
-      gather<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos) { return Conv<S, Re>::ld(stg + pos * M + pl.m); });
-    });
-  } else {
-    const S* in = reinterpret_cast<const S*>(a.in) + bq * a.in_bs1 + br * a.in_bs2 + col;
-    const long long ips = a.in_ps;
-    P.template first<false>([&](auto rc) {
-      constexpr int RR = decltype(rc)::value;
-      gather<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos) {
-        return valid ? Conv<S, Re>::ld(in + pos * ips) : mk<Re>(0.f, 0.f);
-      });
-    });
-  }
-  P.template run<INV, false>(v, pl, sm, tw);
-  S* out = reinterpret_cast<S*>(a.out) + bq * a.out_bs1 + br * a.out_bs2;
-  const Re s = a.scale;
-  if constexpr (MODE == 0) {
-    const long long ops = a.out_ps;
-    P.template last<false>([&](auto rc) {
-      constexpr int RR = decltype(rc)::value;
-      each_natural<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos, Cx<Re> val) {
-        if (valid) Conv<S, Re>::st(out + col + pos * ops, scale(val, s));
-      });
-    });
-  } else {
-    // W_N^{b0 k1}: b0 < N0 and k1 = pos < N1, so the exponent is below N.
-    // Columns past the last one of a partial tile (col >= ncols) take b0 = 0:
-    // their products would index past the table's N entries
-    const Cx<Re>* twl = reinterpret_cast<const Cx<Re>*>(a.twl);
-    const int b0 = a.tw_from_batch ? (int)br : (valid ? col : 0);
-    if constexpr (MODE == 1) {
-      const long long ops = a.out_ps;
-      P.template last<false>([&](auto rc) {
-        constexpr int RR = decltype(rc)::value;
-        each_natural<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos, Cx<Re> val) {
-          const Cx<Re> w = ldg(twl + b0 * pos);
-          if (valid) Conv<S, Re>::st(out + col + pos * ops, scale(INV ? cmulc(val, w) : cmul(val, w), s));
-        });
-      });
-    } else {
-      const int ld = n + 1;  // odd row pitch: the column-major writes below spread over the banks
-      __syncthreads();       // every exchange of the passes is finished with sm
-      P.template last<false>([&](auto rc) {
-        constexpr int RR = decltype(rc)::value;
-        each_natural<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos, Cx<Re> val) {
-          const Cx<Re> w = ldg(twl + b0 * pos);
-          sm[pl.m * ld + pos] = scale(INV ? cmulc(val, w) : cmul(val, w), s);
-        });
-      });
-      __syncthreads();
-      const long long ocs = a.out_cs;
-      const int total = n * M;
-      for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-        const int mm = idx / n, pos = idx - mm * n;
-        const int c = tile * M + mm;
-        if (c < a.ncols) Conv<S, Re>::st(out + c * ocs + pos, sm[mm * ld + pos]);
-      }
-    }
-  }
-}
-
-template <class Plan, class S, int TMA>
-cudaError_t launch_mode(const CUtensorMap& m, const FsArgs& a, const TmaTile& tt, const Launch& l, bool inv,
-                        int mode) {
-  switch (mode * 2 + (inv ? 1 : 0)) {
-    case 0: return enqueue(k_fs<Plan, false, S, 0, TMA>, l, m, a, tt);
-    case 1: return enqueue(k_fs<Plan, true, S, 0, TMA>, l, m, a, tt);
-    case 2: return enqueue(k_fs<Plan, false, S, 1, TMA>, l, m, a, tt);
-    case 3: return enqueue(k_fs<Plan, true, S, 1, TMA>, l, m, a, tt);
-    case 4: return enqueue(k_fs<Plan, false, S, 2, TMA>, l, m, a, tt);
-    default: return enqueue(k_fs<Plan, true, S, 2, TMA>, l, m, a, tt);
-  }
-}
-
-template <class S, int TMA>
-cudaError_t launch_store(const CUtensorMap& m, const FsArgs& a, const TmaTile& tt, const Launch& l, bool inv,
-                         int mode) {
-  const int n = a.pp.n, T = a.pp.T;
-  if constexpr (TMA > 0) {  // staged passes exist for the 128-point short transforms only
-    if (n == 128 && T == 8) return launch_mode<FixPlan<128, 8, RList<16, 8>>, S, TMA>(m, a, tt, l, inv, mode);
-    return cudaErrorInvalidValue;
-  } else {
-    if (n == 128 && T == 8) return launch_mode<FixPlan<128, 8, RList<16, 8>>, S, 0>(m, a, tt, l, inv, mode);
-    if (n == 256 && T == 16) return launch_mode<FixPlan<256, 16, RList<16, 16>>, S, 0>(m, a, tt, l, inv, mode);
-    if (n == 64 && T == 4) return launch_mode<FixPlan<64, 4, RList<16, 4>>, S, 0>(m, a, tt, l, inv, mode);
-    return launch_mode<DynPlan<16>, S, 0>(m, a, tt, l, inv, mode);
-  }
-}
-
-template <class S>
-cudaError_t launch_any(const CUtensorMap& m, const FsArgs& a, const TmaTile& tt, const Launch& l, bool inv,
-                       int mode) {
-  if constexpr (sizeof(S) == 4) {
-    switch (tt.rank) {
-      case 2: return launch_store<S, 2>(m, a, tt, l, inv, mode);
-      case 3: return launch_store<S, 3>(m, a, tt, l, inv, mode);
-      case 4: return launch_store<S, 4>(m, a, tt, l, inv, mode);
-      default: break;
-    }
-  }
-  return launch_store<S, 0>(m, a, tt, l, inv, mode);
-}
 
 // cuTensorMapEncodeTiled, fetched once from the driver without linking libcuda
 PFN_cuTensorMapEncodeTiled_v12000 encoder() {
@@ -322,9 +123,9 @@ cudaError_t launch_fourstep_pass(const FsArgs& a, const Launch& l, int store, bo
     tt.rank = 0;
   }
   switch (store) {
-    case ST_C64: return launch_any<Cx<float>>(map, a, tt, lt, inv, mode);
-    case ST_C32: return launch_any<c32s>(map, a, tt, lt, inv, mode);
-    case ST_BF16: return launch_any<bf16c>(map, a, tt, lt, inv, mode);
+    case ST_C64: return launch_fs_c64(map, a, tt, lt, inv, mode);
+    case ST_C32: return launch_fs_c32(map, a, tt, lt, inv, mode);
+    case ST_BF16: return launch_fs_bf16(map, a, tt, lt, inv, mode);
     default: return cudaErrorInvalidValue;
   }
 }

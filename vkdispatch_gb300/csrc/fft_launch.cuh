@@ -20,21 +20,20 @@ inline bool conv_prefetch() {
 
 // C2C with an optional fused element-wise operation (complex64 only):
 // variant 0 = none, 1 = input weight, 2 = weighted |out|^2 partials
-template <class Plan, bool INV, class S, class Re>
-cudaError_t launch_c2c(const FftArgs& a, const Launch& l, bool strided, int variant) {
+template <class Plan, bool INV, bool STRIDED, class S, class Re>
+cudaError_t launch_c2c_layout(const FftArgs& a, const Launch& l, int variant) {
   if constexpr (std::is_same<S, Cx<float>>::value) {
-    if (variant == 1) {
-      if (strided) return enqueue_pdl(k_c2c<Plan, INV, true, S, Re, 1, 0>, l, a);
-      return enqueue_pdl(k_c2c<Plan, INV, false, S, Re, 1, 0>, l, a);
-    }
-    if (variant == 2) {
-      if (strided) return enqueue_pdl(k_c2c<Plan, INV, true, S, Re, 0, 1>, l, a);
-      return enqueue_pdl(k_c2c<Plan, INV, false, S, Re, 0, 1>, l, a);
-    }
+    if (variant == 1) return enqueue_pdl(k_c2c<Plan, INV, STRIDED, S, Re, 1, 0>, l, a);
+    if (variant == 2) return enqueue_pdl(k_c2c<Plan, INV, STRIDED, S, Re, 0, 1>, l, a);
   }
   if (variant != 0) return cudaErrorInvalidValue;
-  if (strided) return enqueue_pdl(k_c2c<Plan, INV, true, S, Re>, l, a);
-  return enqueue_pdl(k_c2c<Plan, INV, false, S, Re>, l, a);
+  return enqueue_pdl(k_c2c<Plan, INV, STRIDED, S, Re>, l, a);
+}
+
+template <class Plan, bool INV, class S, class Re>
+cudaError_t launch_c2c(const FftArgs& a, const Launch& l, bool strided, int variant) {
+  if (strided) return launch_c2c_layout<Plan, INV, true, S, Re>(a, l, variant);
+  return launch_c2c_layout<Plan, INV, false, S, Re>(a, l, variant);
 }
 
 // convolution with optional spectrum output (complex64 only): variant 0 =
@@ -99,6 +98,8 @@ cudaError_t launch_conv_any(const FftArgs& a, const Launch& l, bool strided, int
 // translation units (C2C, convolution, real) so they compile in parallel.
 template <class S, class Re>
 cudaError_t launch_dyn_c2c(const FftArgs& a, const Launch& l, int op, bool strided, int variant);
+template <class S, class Re, bool STRIDED>
+cudaError_t launch_dyn_c2c_layout(const FftArgs& a, const Launch& l, int op, int variant);
 template <class S, class Re>
 cudaError_t launch_dyn_conv(const FftArgs& a, const Launch& l, bool strided, int kop, int variant);
 template <class S, class Re, bool STRIDED>

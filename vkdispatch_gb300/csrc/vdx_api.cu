@@ -105,6 +105,38 @@ int build_stage_table(int dev, const std::vector<int>& radices, bool f64, void**
   return VDX_OK;
 }
 
+// four-step twiddles (launch_cross_twiddle), one per (device, split)
+std::map<std::tuple<int, int, int>, void*> g_cross_tabs;
+
+int build_cross_table(int dev, int N1, int N0, void** out) {
+  std::lock_guard<std::mutex> lock(g_tab_mu);
+  auto key = std::make_tuple(dev, N1, N0);
+  auto it = g_cross_tabs.find(key);
+  if (it != g_cross_tabs.end()) {
+    *out = it->second;
+    return VDX_OK;
+  }
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, size_t(N1) * size_t(N0) * 8);
+  if (e != cudaSuccess) return fail(VDX_ERR_NOMEM, std::string("twiddle table allocation: ") + cudaGetErrorString(e));
+  cudaStream_t s;
+  e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e != cudaSuccess) {
+    cudaFree(p);
+    return cuda_fail(e, "twiddle stream");
+  }
+  e = launch_cross_twiddle(p, N1, N0, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaStreamDestroy(s);
+  if (e != cudaSuccess) {
+    cudaFree(p);
+    return cuda_fail(e, "twiddle table build");
+  }
+  g_cross_tabs[key] = p;
+  *out = p;
+  return VDX_OK;
+}
+
 std::vector<int> radix_list(const PassPlan& pp) { return std::vector<int>(pp.radix, pp.radix + pp.npass); }
 
 int store_of(int t) {
@@ -132,10 +164,78 @@ namespace vdx {
 // ---------------------------------------------------------------------------
 // radix factorisation
 // ---------------------------------------------------------------------------
-// Splits n into passes: radix 16 for each 2^4, the leftover power of two
-// (2, 4 or 8), 9 for pairs of 3s, then 3, 5, 7, 11, 13.  Fails for primes above 13, the reference's largest
-// supported prime (vkdispatch/fft/prime_utils.py:9-10).
-bool factor_radices(int n, int maxe, std::vector<int>& radices, std::string& why) {
+namespace {
+
+// Threads of one transform: every pass's butterflies fit the threads' points
+// (16 complex registers, floor(16 / R) butterflies of radix R each).
+int threads_of(int n, const std::vector<int>& radices) {
+  int T = 1;
+  for (int r : radices) {
+    const int per = std::max(1, 16 / r);
+    T = std::max(T, (n / r + per - 1) / per);
+  }
+  return T;
+}
+
+// Arithmetic instructions per point of a radix-R butterfly, plus what a pass
+// costs besides (its shared-memory exchange, twiddles and index arithmetic):
+// a pass costs more than most butterflies, so few large radices win
+// (16001 rows of 1500 points: 169.0 us as 5x5x5x4x3, 135.9 us as 15x10x10).
+constexpr double kPassCost = 13.0;
+double radix_cost(int r) {
+  static const double c[17] = {0,   0,   2.0,  4.7, 4.0,  7.2, 6.7,  9.4, 7.0,
+                               11., 9.2, 13.6, 8.7, 15.7, 11.4, 11.9, 10.0};
+  return kPassCost + c[r];
+}
+
+struct RadixSearch {
+  int n, tmax;
+  std::vector<int> cur, best;
+  double best_cost = 1e30;
+  int best_t = 0;
+
+  // rem = product still to place, in radices of at most rmax
+  void go(int rem, int rmax, double cost) {
+    if (rem == 1) {
+      const int t = threads_of(n, cur);
+      // even radices only: the first scatter's stride conflicts in the banks
+      if (std::none_of(cur.begin(), cur.end(), [](int r) { return r % 2 == 1; })) cost += 2.0;
+      const bool fits = t <= tmax, best_fits = !best.empty() && best_t <= tmax;
+      // a list whose threads fit the CTA beats every one whose do not
+      const bool better = best.empty() || (fits != best_fits ? fits
+                                           : fits           ? (cost < best_cost - 1e-9 ||
+                                                     (cost < best_cost + 1e-9 && t < best_t))
+                                                            : t < best_t);
+      if (better) {
+        best = cur;
+        best_cost = cost;
+        best_t = t;
+      }
+      return;
+    }
+    if ((int)cur.size() >= kMaxPasses) return;
+    // no list costs less than radix 16's 23 instructions per four bits
+    if (!best.empty() && best_t <= tmax && cost + 5.75 * std::log2(double(rem)) > best_cost) return;
+    for (int r = rmax; r >= 2; --r) {
+      if (rem % r) continue;
+      cur.push_back(r);
+      go(rem / r, r, cost + radix_cost(r));
+      cur.pop_back();
+    }
+  }
+};
+
+}  // namespace
+
+// Splits n into radix passes.  Powers of two (whose compile-time plans name
+// their lists) and fp64 plans (8 points per thread): radix 16 (8) for each 2^4
+// (2^3), then the leftover power of two, 9 for pairs of 3s, then 3, 5, 7, 11,
+// 13.  Every other fp32 length up to one CTA's 16384 points: the cheapest list
+// of radices 2..16 whose threads fit in tmax, an odd radix first where there
+// is one (its stride-R scatter does not bank-conflict).  Fails for primes
+// above 13, the reference's largest supported prime
+// (vkdispatch/fft/prime_utils.py:9-10).
+bool factor_radices(int n, int maxe, std::vector<int>& radices, std::string& why, int tmax) {
   radices.clear();
   if (n == 1) {
     radices.push_back(1);
@@ -185,6 +285,23 @@ bool factor_radices(int n, int maxe, std::vector<int>& radices, std::string& why
     return false;
   }
   std::sort(radices.begin(), radices.end(), [](int x, int y) { return x > y; });
+  if (maxe == 16 && (n & (n - 1)) != 0 && n <= 16384) {
+    // found lists are kept: a batch of long items asks for every divisor
+    static std::mutex mu;
+    static std::map<std::pair<int, int>, std::vector<int>> found;
+    std::lock_guard<std::mutex> lock(mu);
+    std::vector<int>& best = found[{n, tmax}];
+    if (best.empty()) {
+      RadixSearch s;
+      s.n = n;
+      s.tmax = tmax;
+      s.go(n, 16, 0.0);
+      best = s.best;
+    }
+    radices = best;
+    auto odd = std::find_if(radices.begin(), radices.end(), [](int r) { return r % 2 == 1; });
+    if (odd != radices.end()) std::rotate(radices.begin(), odd, odd + 1);
+  }
   return true;
 }
 
@@ -193,6 +310,8 @@ int get_twiddle_table(int dev, int count, int den, bool f64, void** out) { retur
 int get_stage_table(int dev, const std::vector<int>& radices, bool f64, void** out) {
   return build_stage_table(dev, radices, f64, out);
 }
+
+int get_cross_table(int dev, int N1, int N0, void** out) { return build_cross_table(dev, N1, N0, out); }
 
 int set_error(int code, const char* msg) { return fail(code, msg); }
 
@@ -300,7 +419,7 @@ namespace {
 
 int sub_pass_plan(int n, int M, PassPlan& pp, std::string& why) {
   std::vector<int> r;
-  if (!factor_radices(n, 16, r, why)) return VDX_ERR_UNSUPPORTED;
+  if (!factor_radices(n, 16, r, why, 512)) return VDX_ERR_UNSUPPORTED;
   std::memset(&pp, 0, sizeof(pp));
   pp.n = n;
   pp.npass = (int)r.size();
@@ -522,7 +641,10 @@ int plan_fourstep(vdx_plan* p, long long inner, long long outer, int smem_optin)
   };
   int rc = short_table(ppA, &p->fsA.tw);
   if (rc == VDX_OK) rc = short_table(ppB, &p->fsB.tw);
-  if (rc == VDX_OK) rc = get_table(p->dev, N, N, false, const_cast<void**>(&p->fsA.twl));
+  if (rc == VDX_OK)
+    rc = p->tensor_core ? get_table(p->dev, N, N, false, const_cast<void**>(&p->fsA.twl))
+                        : build_cross_table(p->dev, N1, N0, const_cast<void**>(&p->fsA.twl));
+  p->fsA.tw_ld = N0;
   if (rc != VDX_OK) return rc;
   p->fsA.scale = 1.f;
   p->fsB.scale = float(p->args.scale);
@@ -593,8 +715,8 @@ int plan_conv2d_real(const vdx_fft_desc& d, vdx_plan** plan) {
   // the kernel's compile-time plans of W/2 and H points (fft_conv2d.cu)
   std::vector<int> rrow, rcol;
   std::string why;
-  factor_radices(W / 2, 16, rrow, why);
-  factor_radices(H, 16, rcol, why);
+  factor_radices(W / 2, 16, rrow, why, 1024);
+  factor_radices(H, 16, rcol, why, 1024);
   int rc = build_stage_table(p->dev, rrow, false, &t);
   c.tw_row = static_cast<const Cx<float>*>(t);
   if (rc == VDX_OK) rc = get_table(p->dev, W / 2 + 1, W, false, &t);
@@ -926,7 +1048,7 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
   }
   const int maxe = f64 ? MaxE<double>::value : (pmaxe == 8 ? 8 : MaxE<float>::value);
   std::string why;
-  if (!factor_radices(n, maxe, p->radices, why)) {
+  if (!factor_radices(n, maxe, p->radices, why, 1024)) {
     delete p;
     if ((d.flags & VDX_FFT_FLAG_BLUESTEIN) && d.kind == VDX_KIND_C2C && lo == 0 && hi == N)
       return plan_bluestein(d, inner, outer, N, st, f64, plan);
@@ -1026,6 +1148,7 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
   a.pp.M = M;
   a.pp.npad = npad;
   set_pass_tables(a.pp);
+  if (is_conv) a.pp.pad = 0;  // the reversed list steps differently
   a.sig_lo = lo;
   a.sig_hi = hi;
   a.nreal = N;

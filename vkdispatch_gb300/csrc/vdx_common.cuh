@@ -319,16 +319,59 @@ struct DftComposite {
   };
 };
 
+// Composite R = A*B with coprime A and B (Good-Thomas prime-factor split): with
+// n = (B a + A b) mod R and k = the residue with k = ka mod A, k = kb mod B,
+// W_R^{nk} = W_A^{a ka} W_B^{b kb}, so no twiddles lie between the two halves
+// and both index maps are register renamings.
+template <int R, int A, bool INV, class Re>
+struct DftCoprime {
+  static constexpr int B = R / A;
+  static constexpr int residue(int ka, int kb) {
+    int k = 0;
+    while (k % A != ka || k % B != kb) ++k;
+    return k;
+  }
+  template <int I>
+  static __device__ __forceinline__ void columns(Cx<Re> (&z)[A][B], Cx<Re>* v) {
+    Cx<Re> t[A];
+#pragma unroll
+    for (int a = 0; a < A; ++a) t[a] = z[a][I];
+    Dft<A, INV, Re>::run(t);
+    put<I, 0>(t, v);
+    if constexpr (I + 1 < B) columns<I + 1>(z, v);
+  }
+  template <int KB, int KA>
+  static __device__ __forceinline__ void put(const Cx<Re>* t, Cx<Re>* v) {
+    constexpr int k = residue(KA, KB);
+    v[k] = t[KA];
+    if constexpr (KA + 1 < A) put<KB, KA + 1>(t, v);
+  }
+  static __device__ __forceinline__ void run(Cx<Re>* v) {
+    Cx<Re> z[A][B];
+#pragma unroll
+    for (int a = 0; a < A; ++a)
+#pragma unroll
+      for (int b = 0; b < B; ++b) z[a][b] = v[(B * a + A * b) % R];
+#pragma unroll
+    for (int a = 0; a < A; ++a) Dft<B, INV, Re>::run(z[a]);
+    columns<0>(z, v);
+  }
+};
+
 template <bool INV, class Re>
-struct Dft<6, INV, Re> : DftComposite<6, 2, INV, Re> {};
+struct Dft<6, INV, Re> : DftCoprime<6, 2, INV, Re> {};
 template <bool INV, class Re>
 struct Dft<8, INV, Re> : DftComposite<8, 2, INV, Re> {};
 template <bool INV, class Re>
 struct Dft<9, INV, Re> : DftComposite<9, 3, INV, Re> {};
 template <bool INV, class Re>
-struct Dft<10, INV, Re> : DftComposite<10, 2, INV, Re> {};
+struct Dft<10, INV, Re> : DftCoprime<10, 2, INV, Re> {};
 template <bool INV, class Re>
-struct Dft<12, INV, Re> : DftComposite<12, 4, INV, Re> {};
+struct Dft<12, INV, Re> : DftCoprime<12, 4, INV, Re> {};
+template <bool INV, class Re>
+struct Dft<14, INV, Re> : DftCoprime<14, 2, INV, Re> {};
+template <bool INV, class Re>
+struct Dft<15, INV, Re> : DftCoprime<15, 3, INV, Re> {};
 template <bool INV, class Re>
 struct Dft<16, INV, Re> : DftComposite<16, 4, INV, Re> {};
 template <bool INV, class Re>

@@ -37,6 +37,16 @@ struct MaxE<double> {
   static constexpr int value = 8;
 };
 
+// Runtime-radix plan of a (storage, compute) pair: rows step linearly through
+// their shared-memory slots in fp32, where the planner puts an odd radix first
+// or the list is 16s and one last radix.  fp64 lists (radix 8) and the
+// convolutions of 16-bit storage, whose powers of two have no compile-time
+// plan and run their lists in both orders, compute every padded slot.
+template <class S, class Re>
+using DynPlanOf = DynPlan<MaxE<Re>::value, !Same<Re, float>::value>;
+template <class S, class Re>
+using DynConvPlanOf = DynPlan<MaxE<Re>::value, !Same<S, Cx<float>>::value>;
+
 // Supported (storage, compute) pairs: complex64/fp32, complex32/fp32,
 // bf16x2/fp32, complex128/fp64.
 enum Op { OP_C2C_FWD, OP_C2C_INV, OP_CONV, OP_R2C_EVEN, OP_C2R_EVEN, OP_R2C_ODD, OP_C2R_ODD, OP_CONV2D_REAL };
@@ -51,6 +61,11 @@ template <class S, class Re>
 cudaError_t launch_dyn_real(const FftArgs& a, const Launch& l, int op);
 
 cudaError_t launch_twiddle(void* tab, int count, int den, bool f64, cudaStream_t s);
+// Four-step twiddles laid out like the intermediate: tab[k1 * N0 + b0] =
+// W_{N1 N0}^{b0 k1}, so that a tile's lanes (neighbouring b0) read neighbouring
+// entries; in a natural table W_N^i every lane's entry b0 k1 lies on a sector
+// of its own.
+cudaError_t launch_cross_twiddle(void* tab, int N1, int N0, cudaStream_t s);
 cudaError_t launch_stage_twiddle(void* tab, const PassPlan& pp, bool f64, cudaStream_t s);
 
 // One pass of a four-step long-axis transform (fft_large.cu): tiles of M
@@ -63,7 +78,8 @@ struct FsArgs {
   const void* in;
   void* out;
   const void* tw;   // stage-ordered twiddles of the short transform (tensor-core passes: W_n^k)
-  const void* twl;  // W_N^k of the whole axis (pass A)
+  const void* twl;  // pass A: cross twiddles W_N^{b0 k1} at k1 * tw_ld + b0 (tensor-core passes: W_N^k)
+  int tw_ld;
   long long split;
   long long in_bs1, in_bs2, out_bs1, out_bs2;
   long long in_ps, out_ps, out_cs;
