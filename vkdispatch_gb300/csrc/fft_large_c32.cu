@@ -2,8 +2,7 @@
 #include "fft_large.cuh"
 
 namespace vdx {
-cudaError_t launch_fs_c32(const CUtensorMap& m, const FsArgs& a, const TmaTile& tt, const Launch& l, bool inv,
-                        int mode) {
-  return launch_any<c32s>(m, a, tt, l, inv, mode);
+cudaError_t launch_fs_c32(const FsArgs& a, const Launch& l, bool inv, int mode) {
+  return launch_any<c32s>(a, l, inv, mode);
 }
 }  // namespace vdx

@@ -735,16 +735,6 @@ int plan_conv2d_real(const vdx_fft_desc& d, vdx_plan** plan) {
   return VDX_OK;
 }
 
-// Four-step passes of strided axes stage their input tiles with TMA tensor
-// copies where fourstep_tma_ok allows it, unless VDX_FOURSTEP_TMA=0.
-bool fourstep_tma() {
-  static const bool on = [] {
-    const char* e = std::getenv("VDX_FOURSTEP_TMA");
-    return !(e && e[0] == '0');
-  }();
-  return on;
-}
-
 cudaError_t exec_fourstep(const vdx_plan* p, const void* in, void* out, cudaStream_t s) {
   if (p->fused) {
     FusedLaunch fl = p->fl;
@@ -781,10 +771,9 @@ cudaError_t exec_fourstep(const vdx_plan* p, const void* in, void* out, cudaStre
         A.col_tiles = (int)((Cc + MA - 1) / MA);
         A.tw_from_batch = 1;
         A.nbatch = Oc * N0;
-        A.status = p->d_status;
         la.grid = dim3((unsigned)(Oc * N0 * A.col_tiles));
         e = p->tensor_core ? launch_fourstep_pass_tc(A, la, p->store, inv, 1, p->tc_bmat, p->d_status)
-                           : launch_fourstep_pass(A, la, p->store, inv, 1, fourstep_tma());
+                           : launch_fourstep_pass(A, la, p->store, inv, 1);
         if (e != cudaSuccess) return e;
         FsArgs B = p->fsB;
         B.in = p->ws;
@@ -800,10 +789,9 @@ cudaError_t exec_fourstep(const vdx_plan* p, const void* in, void* out, cudaStre
         B.ncols = (int)Cc;
         B.col_tiles = (int)((Cc + MB - 1) / MB);
         B.nbatch = Oc * N1;
-        B.status = p->d_status;
         lb.grid = dim3((unsigned)(Oc * N1 * B.col_tiles));
         e = p->tensor_core ? launch_fourstep_pass_tc(B, lb, p->store, inv, 0, p->tc_bmat, p->d_status)
-                           : launch_fourstep_pass(B, lb, p->store, inv, 0, fourstep_tma());
+                           : launch_fourstep_pass(B, lb, p->store, inv, 0);
         if (e != cudaSuccess) return e;
       }
     }
@@ -827,10 +815,9 @@ cudaError_t exec_fourstep(const vdx_plan* p, const void* in, void* out, cudaStre
     A.col_tiles = (int)((N0 + MA - 1) / MA);
     A.tw_from_batch = 0;
     A.nbatch = Rr;
-    A.status = p->d_status;
     la.grid = dim3((unsigned)(Rr * A.col_tiles));
     e = p->tensor_core ? launch_fourstep_pass_tc(A, la, p->store, inv, 2, p->tc_bmat, p->d_status)
-                       : launch_fourstep_pass(A, la, p->store, inv, 2, false);
+                       : launch_fourstep_pass(A, la, p->store, inv, 2);
     if (e != cudaSuccess) return e;
     FsArgs B = p->fsB;
     B.in = p->ws;
@@ -846,10 +833,9 @@ cudaError_t exec_fourstep(const vdx_plan* p, const void* in, void* out, cudaStre
     B.ncols = (int)N1;
     B.col_tiles = (int)((N1 + MB - 1) / MB);
     B.nbatch = Rr;
-    B.status = p->d_status;
     lb.grid = dim3((unsigned)(Rr * B.col_tiles));
     e = p->tensor_core ? launch_fourstep_pass_tc(B, lb, p->store, inv, 0, p->tc_bmat, p->d_status)
-                       : launch_fourstep_pass(B, lb, p->store, inv, 0, false);
+                       : launch_fourstep_pass(B, lb, p->store, inv, 0);
     if (e != cudaSuccess) return e;
   }
   return e;
@@ -1114,7 +1100,12 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
   int M = 1;
   size_t smem = 0;
   if (strided) {
-    int mcols = 8;
+    // columns per tile: 8 (64-byte row segments of complex64), 16 where a
+    // column has at most 16 threads, so that CTAs do not get small
+    // (256^3 along axis 0: 53.2 us with 8, 49.2 with 16, 52.8 with 32;
+    // 1024 x 96 x 170: 57.9, 52.5, 57.3; but 64 x 512 x 512: 55.7, 62.9, 71.3
+    // and 16 x 1024 x 1024: 69.2, 76.3)
+    int mcols = !f64 && pmaxe == 16 && T <= 16 ? 16 : 8;
     if (const char* e = std::getenv("VDX_STRIDED_COLUMNS")) mcols = std::max(1, std::min(32, std::atoi(e)));
     if (tune.width > 0) mcols = std::min(32, tune.width);
     M = (int)std::min<long long>(mcols, inner);
@@ -1123,7 +1114,10 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
     smem = need_smem ? size_t(n) * M * cbytes : 0;
   } else {
     const long long ntrans = outer;
-    int cta_threads = 128;
+    // rows per CTA: about 64 threads, since transforms that span warps share
+    // the CTA's barriers (100000 x 360: 150 us with 128 threads, 138 with 64;
+    // transforms inside one warp are indifferent)
+    int cta_threads = 64;
     if (const char* e = std::getenv("VDX_CTA_THREADS")) cta_threads = std::max(32, std::min(1024, std::atoi(e)));
     if (tune.width > 0) cta_threads = std::max(32, std::min(1024, tune.width));
     M = std::max(1, cta_threads / T);
