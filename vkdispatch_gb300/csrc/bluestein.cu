@@ -8,11 +8,12 @@
 //   a[m] = x[m] w[m] (m < N), 0 otherwise;
 //   b[m] = conj(w[m]) for m < N, b[M - m] = conj(w[m]) for 0 < m < N, 0 otherwise;
 //   X[k] = w[k] * IFFT_M(FFT_M(a) * FFT_M(b))[k].
-// The middle step is one fused convolution launch (k_conv multiplies by the
-// conjugate of its kernel, so the kernel passed is conj(FFT_M(b))) while M
-// fits one CTA per transform; longer M run it as a four-step forward
-// transform, a spectrum product (k_bs_mul) and a four-step inverse.  The chirp
-// is built in FP64 from the exact integer n^2 mod 2N, so no angle grows with n.
+// While M fits one CTA per transform all of it is one launch (k_bluestein,
+// fft_kernels.cuh), which multiplies by the conjugate of its kernel, so the
+// kernel passed is conj(FFT_M(b)).  Longer M run chirp-in into a padded
+// workspace, a four-step forward transform, a spectrum product (k_bs_mul), a
+// four-step inverse and chirp-out.  The chirp is built in FP64 from the exact
+// integer n^2 mod 2N, so no angle grows with n.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -107,6 +107,14 @@ cudaError_t launch_dyn_conv_layout(const FftArgs& a, const Launch& l, int kop, i
 template <class S, class Re>
 cudaError_t launch_dyn_real(const FftArgs& a, const Launch& l, int op);
 
+template <class Plan, class S, class Re>
+cudaError_t launch_bluestein(const FftArgs& a, const Launch& l, bool strided) {
+  if (strided) return enqueue_pdl(k_bluestein<Plan, true, S, Re>, l, a);
+  return enqueue_pdl(k_bluestein<Plan, false, S, Re>, l, a);
+}
+template <class S, class Re>
+cudaError_t launch_dyn_bluestein(const FftArgs& a, const Launch& l, bool strided);
+
 template <class Plan, class S, class Re, bool WITH_ODD>
 cudaError_t launch_with_plan(const FftArgs& a, const Launch& l, int op, bool strided, int kop, int variant) {
   if (variant != 0 && op != OP_C2C_FWD && op != OP_C2C_INV && op != OP_CONV) return cudaErrorInvalidValue;
@@ -116,6 +124,8 @@ cudaError_t launch_with_plan(const FftArgs& a, const Launch& l, int op, bool str
       return launch_c2c_any<Plan, S, Re>(a, l, op, strided, variant);
     case OP_CONV:
       return launch_conv_any<Plan, S, Re>(a, l, strided, kop, variant);
+    case OP_BLUESTEIN:
+      return launch_bluestein<Plan, S, Re>(a, l, strided);
     default:
       return launch_real<Plan, S, Re>(a, l, op, WITH_ODD);
   }
@@ -130,6 +140,8 @@ cudaError_t launch_fft(const FftArgs& a, const Launch& l, int op, bool strided, 
       return launch_dyn_c2c<S, Re>(a, l, op, strided, variant);
     case OP_CONV:
       return launch_dyn_conv<S, Re>(a, l, strided, kop, variant);
+    case OP_BLUESTEIN:
+      return launch_dyn_bluestein<S, Re>(a, l, strided);
     default:
       return launch_dyn_real<S, Re>(a, l, op);
   }

@@ -847,7 +847,8 @@ namespace {
 
 int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan);
 
-// Bluestein plan (bluestein.cu): three launches per execution.
+// Bluestein plan (bluestein.cu): one launch per execution while the
+// convolution fits one CTA, else chirp launches around two long transforms.
 int plan_bluestein(const vdx_fft_desc& d, long long inner, long long outer, int N, int st, bool f64,
                    vdx_plan** plan) {
   int M = 1;
@@ -890,7 +891,9 @@ int plan_bluestein(const vdx_fft_desc& d, long long inner, long long outer, int 
   dc.kernel_broadcast = 1;
   int rc = VDX_OK;
   if (!split) {
-    rc = create_plan(&dc, Tune{}, &p->bs_conv);
+    Tune t;
+    if (st != ST_C64) t.maxe = 16;  // the two-pass radix-32 plans exist for complex64 storage
+    rc = create_plan(&dc, t, &p->bs_conv);
   } else {
     dc.kind = VDX_KIND_C2C;
     dc.normalize = 0;
@@ -911,8 +914,10 @@ int plan_bluestein(const vdx_fft_desc& d, long long inner, long long outer, int 
   cudaStream_t s = nullptr;
   e = cudaMalloc(&p->bs_w, size_t(N) * es);
   if (e == cudaSuccess) e = cudaMalloc(&b, size_t(M) * es);
-  if (e == cudaSuccess) e = cudaMalloc(&p->bs_K, size_t(M) * size_t(inner) * es);
-  if (e == cudaSuccess) e = cudaMalloc(&p->bs_ws, size_t(outer) * size_t(M) * size_t(inner) * es);
+  // the fused kernel reads one spectrum for every column
+  const long long kcols = split ? inner : 1;
+  if (e == cudaSuccess) e = cudaMalloc(&p->bs_K, size_t(M) * size_t(kcols) * es);
+  if (e == cudaSuccess && split) e = cudaMalloc(&p->bs_ws, size_t(outer) * size_t(M) * size_t(inner) * es);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = launch_chirp_tables(p->bs_w, b, N, M, d.inverse ? 1 : -1, f64, s);
   if (e == cudaSuccess) {
@@ -927,7 +932,7 @@ int plan_bluestein(const vdx_fft_desc& d, long long inner, long long outer, int 
     df.signal_lo = df.signal_hi = -1;
     rc = create_plan(&df, Tune{}, &tmp);
     if (rc == VDX_OK) rc = vdx_fft_exec(tmp, b, b, nullptr, s);  // B = FFT_M(b)
-    if (rc == VDX_OK) e = launch_conj_slab(p->bs_K, b, M, inner, f64, s);
+    if (rc == VDX_OK) e = launch_conj_slab(p->bs_K, b, M, kcols, f64, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   }
   delete tmp;
@@ -1622,19 +1627,42 @@ int exec_plan(const vdx_plan* p, const void* in, void* out, const void* kernel, 
     if (ops && (ops->in_weight || ops->spec_out || ops->loss_weight))
       return fail(VDX_ERR_UNSUPPORTED, "fused operations are not available on Bluestein plans");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    if (p->bs_conv) {
+      const vdx_plan* c = p->bs_conv;
+      FftArgs a = c->args;
+      a.in = in;
+      a.out = out;
+      a.ker = p->bs_K;
+      a.in_bs = a.out_bs = (long long)p->N * p->inner;
+      a.chirp = p->bs_w;
+      a.chirp_n = p->N;
+      a.chirp_scale = norm_scale(p->d.normalize, p->N);
+      Launch l = c->launch;
+      l.stream = s;
+      const int n = a.pp.n;
+      if (p->store == ST_C64 && c->fixed_pts)
+        e = launch_fixedpts_c64_any(n, c->fixed_pts, a, l, OP_BLUESTEIN, c->strided, 0, 0);
+      else if (p->store == ST_C64 && c->fixed)
+        e = launch_fixed_c64_any(n, a, l, OP_BLUESTEIN, c->strided, 0, 0);
+      else if (p->store == ST_C64)
+        e = launch_fft<Cx<float>, float>(a, l, OP_BLUESTEIN, c->strided, 0, 0);
+      else if (p->store == ST_C32)
+        e = launch_fft<c32s, float>(a, l, OP_BLUESTEIN, c->strided, 0, 0);
+      else if (p->store == ST_BF16)
+        e = launch_fft<bf16c, float>(a, l, OP_BLUESTEIN, c->strided, 0, 0);
+      else
+        e = launch_fft<Cx<double>, double>(a, l, OP_BLUESTEIN, c->strided, 0, 0);
+      if (e != cudaSuccess) return cuda_fail(e, "Bluestein launch");
+      return VDX_OK;
+    }
     e = launch_bluestein_io(true, p->store, in, p->bs_ws, p->bs_w, p->outer, p->N, p->bs_M, p->inner, 1.0, s);
     if (e != cudaSuccess) return cuda_fail(e, "Bluestein chirp-in launch");
-    if (p->bs_conv) {
-      const int rc = exec_plan(p->bs_conv, p->bs_ws, p->bs_ws, p->bs_K, nullptr, stream);
-      if (rc != VDX_OK) return rc;
-    } else {
-      int rc = exec_plan(p->bs_fwd, p->bs_ws, p->bs_ws, nullptr, nullptr, stream);
-      if (rc != VDX_OK) return rc;
-      e = launch_bluestein_mul(p->bs_ws, p->bs_K, p->outer, p->bs_M, p->inner, p->f64, s);
-      if (e != cudaSuccess) return cuda_fail(e, "Bluestein spectrum product launch");
-      rc = exec_plan(p->bs_inv, p->bs_ws, p->bs_ws, nullptr, nullptr, stream);
-      if (rc != VDX_OK) return rc;
-    }
+    int rc = exec_plan(p->bs_fwd, p->bs_ws, p->bs_ws, nullptr, nullptr, stream);
+    if (rc != VDX_OK) return rc;
+    e = launch_bluestein_mul(p->bs_ws, p->bs_K, p->outer, p->bs_M, p->inner, p->f64, s);
+    if (e != cudaSuccess) return cuda_fail(e, "Bluestein spectrum product launch");
+    rc = exec_plan(p->bs_inv, p->bs_ws, p->bs_ws, nullptr, nullptr, stream);
+    if (rc != VDX_OK) return rc;
     e = launch_bluestein_io(false, p->store, out, p->bs_ws, p->bs_w, p->outer, p->N, p->bs_M, p->inner,
                             norm_scale(p->d.normalize, p->N), s);
     if (e != cudaSuccess) return cuda_fail(e, "Bluestein chirp-out launch");

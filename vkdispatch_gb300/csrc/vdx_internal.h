@@ -49,7 +49,7 @@ using DynConvPlanOf = DynPlan<MaxE<Re>::value, !Same<S, Cx<float>>::value>;
 
 // Supported (storage, compute) pairs: complex64/fp32, complex32/fp32,
 // bf16x2/fp32, complex128/fp64.
-enum Op { OP_C2C_FWD, OP_C2C_INV, OP_CONV, OP_R2C_EVEN, OP_C2R_EVEN, OP_R2C_ODD, OP_C2R_ODD, OP_CONV2D_REAL };
+enum Op { OP_C2C_FWD, OP_C2C_INV, OP_CONV, OP_R2C_EVEN, OP_C2R_EVEN, OP_R2C_ODD, OP_C2R_ODD, OP_CONV2D_REAL, OP_BLUESTEIN };
 
 template <class S, class Re>
 cudaError_t launch_fft(const FftArgs& a, const Launch& l, int op, bool strided, int kop, int variant);
