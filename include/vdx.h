@@ -120,6 +120,15 @@ typedef struct vdx_fft_desc {
  * as in the reference.
  */
 #define VDX_FFT_FLAG_BLUESTEIN 4
+/*
+ * VDX_FFT_FLAG_DENSE_REAL: the real side of an R2C or C2R transform is dense
+ * rows of N reals (C order, N even) instead of the packed layout's N + 2; the
+ * transform runs out of place (in != out) and the real array starts on a
+ * complex element's alignment.  The half spectrum keeps its N/2 + 1 complex
+ * elements per row.  No counterpart in the reference, whose real transforms
+ * are in place on packed rows (vkdispatch/base/buffer.py:377-448).
+ */
+#define VDX_FFT_FLAG_DENSE_REAL 8
 
 typedef struct vdx_plan vdx_plan;
 

@@ -981,8 +981,11 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
       return fail(VDX_ERR_UNSUPPORTED, "VDX_KOP_MUL convolutions need complex64 storage");
   }
   if (real && (st == ST_BF16)) return fail(VDX_ERR_UNSUPPORTED, "real transforms support complex64/complex32/complex128");
-  if (d.flags & ~(VDX_FFT_FLAG_TENSOR_CORE | VDX_FFT_FLAG_AUTOTUNE | VDX_FFT_FLAG_BLUESTEIN))
+  if (d.flags & ~(VDX_FFT_FLAG_TENSOR_CORE | VDX_FFT_FLAG_AUTOTUNE | VDX_FFT_FLAG_BLUESTEIN | VDX_FFT_FLAG_DENSE_REAL))
     return fail(VDX_ERR_INVALID, "unknown bits in desc.flags");
+  const bool dense = (d.flags & VDX_FFT_FLAG_DENSE_REAL) != 0;
+  if (dense && (!real || d.shape[d.axis] % 2 != 0))
+    return fail(VDX_ERR_INVALID, "dense real rows are defined for R2C and C2R transforms of even length");
   if (d.normalize < 0 || d.normalize > 2) return fail(VDX_ERR_INVALID, "normalize must be 0, 1 or 2");
 
   long long inner = 1, outer = 1;
@@ -1188,6 +1191,8 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
     a.ntrans = outer;
     a.inner = 1;
     a.in_bs = a.out_bs = row;
+    // dense rows of N reals are N / 2 complex elements apart
+    if (dense) (d.kind == VDX_KIND_R2C ? a.in_bs : a.out_bs) = N / 2;
     a.ker_bs = d.kernel_broadcast ? 0 : row;
     const long long blocks = (outer + M - 1) / M;
     if (blocks > 0x7fffffffLL) {
@@ -1328,6 +1333,7 @@ int autotune_plan(const vdx_fft_desc& d0, vdx_plan** plan) {
   }
   const long long outer_t = std::min(outer, std::max(1ll, cap / (long long)(row * inner_t * es)));
   vdx_fft_desc dt = d;
+  dt.flags &= ~VDX_FFT_FLAG_DENSE_REAL;  // the search runs in place on packed rows
   if (inner_t > 1) {
     dt.ndim = 3;
     dt.shape[0] = outer_t;
@@ -1619,6 +1625,12 @@ int exec_plan(const vdx_plan* p, const void* in, void* out, const void* kernel, 
     return VDX_OK;
   }
   if (p->op == OP_CONV && !kernel) return fail(VDX_ERR_INVALID, "convolution needs a kernel spectrum");
+  if (p->d.flags & VDX_FFT_FLAG_DENSE_REAL) {
+    if (in == out) return fail(VDX_ERR_INVALID, "dense real transforms run out of place (in != out)");
+    const void* r = p->d.kind == VDX_KIND_R2C ? in : out;
+    if (reinterpret_cast<uintptr_t>(r) % store_bytes(p->store) != 0)
+      return fail(VDX_ERR_INVALID, "dense real rows must start on a complex element's alignment");
+  }
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");

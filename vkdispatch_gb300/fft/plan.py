@@ -138,6 +138,11 @@ class Plan:
             pass
 
 
+def dense_real_flags() -> int:
+    """Plan flags of a real transform whose real side is dense rows."""
+    return L.VDX_FFT_FLAG_DENSE_REAL | (L.VDX_FFT_FLAG_AUTOTUNE if getattr(_tls, "tune", False) else 0)
+
+
 def _default_flags(shape, axis: int, kind: int, io_type: int, compute_type: int, signal_range) -> int:
     """Plan flags from the calling thread's settings (tensor-core stages,
     autotuning, Bluestein)."""
