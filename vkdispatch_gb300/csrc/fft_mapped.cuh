@@ -215,7 +215,13 @@ __device__ __forceinline__ R m_length(R a) {
 
 // MODE 0: forward FFT, 1: inverse FFT, 2: fused convolution (forward FFT,
 // kernel hook, inverse FFT with the passes reversed)
-template <class Plan, bool STRIDED, class Re, int MODE, class H>
+// IO32: every io_index is below 2^32 (the plan knows its shape).  The index
+// then reaches the hooks as a zero-extended 32-bit value, so the divisions and
+// remainders by constant dimensions that index maps consist of
+// (unravel_index(ravel_index(..))) narrow to 32 bits; as 64-bit divisions they
+// cost a tenth of the kernel (16 x 600 x 512 points of a padded correlation:
+// 85.6 us, 80.5 us narrowed).
+template <class Plan, bool STRIDED, class Re, int MODE, class H, bool IO32 = false>
 __device__ __forceinline__ void mapped_body(const FftArgs& a, const MapArgs& m) {
   const Plan P(a.pp);
   constexpr int MAXE = Plan::MAXE;
@@ -227,13 +233,17 @@ __device__ __forceinline__ void mapped_body(const FftArgs& a, const MapArgs& m) 
   P.assume_t(pl.t);
   const int n = P.n();
   const long long io0 = pl.in0();
+  auto io_at = [&](int pos) -> long long {
+    if constexpr (IO32) return (long long)(unsigned(io0) + unsigned(pos) * unsigned(pl.ps));
+    else return io0 + pos * pl.ps;
+  };
   const bool ok = pl.tile_full || pl.valid;
   const int lo = a.sig_lo, hi = a.sig_hi;
   P.template first<false>([&](auto rc) {
     constexpr int RR = decltype(rc)::value;
     gather<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos) {
       if (!ok || pos < lo || pos >= hi) return mk<Re>(Re(0), Re(0));
-      return H::template load<Re>(m, io0 + pos * pl.ps, pos, n);
+      return H::template load<Re>(m, io_at(pos), pos, n);
     });
   });
   P.template run<MODE == 1, false>(v, pl, sm, tw);
@@ -250,7 +260,7 @@ __device__ __forceinline__ void mapped_body(const FftArgs& a, const MapArgs& m) 
 #pragma unroll
           for (int r = 0; r < RR; ++r) {
             const int pos = j + r * nb;
-            v[b * RR + r] = H::template kernel<Re>(m, v[b * RR + r], io0 + pos * pl.ps, pos, n);
+            v[b * RR + r] = H::template kernel<Re>(m, v[b * RR + r], io_at(pos), pos, n);
           }
         }
       }
@@ -261,7 +271,7 @@ __device__ __forceinline__ void mapped_body(const FftArgs& a, const MapArgs& m) 
   P.template last<REV>([&](auto rc) {
     constexpr int RR = decltype(rc)::value;
     each_natural<RR, MAXE, Re>(v, n / RR, P.T(), pl.t, [&](int pos, Cx<Re> val) {
-      if (ok) H::template store<Re>(m, scale(val, s), io0 + pos * pl.ps, pos, n);
+      if (ok) H::template store<Re>(m, scale(val, s), io_at(pos), pos, n);
     });
   });
 }

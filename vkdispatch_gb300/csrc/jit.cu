@@ -203,6 +203,8 @@ int vdx_map_plan_create(const vdx_fft_desc* desc, const char* hooks_source, vdx_
   const MapGeometry& g = p->g;
   const int mode = desc->kind == VDX_KIND_CONV ? 2 : (desc->inverse ? 1 : 0);
   const int maxe = g.f64 ? MaxE<double>::value : MaxE<float>::value;
+  long long total = 1;  // io_index < total
+  for (int i = 0; i < d.ndim; ++i) total *= d.shape[i];
   std::string radices;
   for (size_t i = 0; i < g.radices.size(); ++i) radices += (i ? ", " : "") + std::to_string(g.radices[i]);
   p->source = std::string("#include \"fft_mapped.cuh\"\n\n") + hooks_source +
@@ -210,7 +212,7 @@ int vdx_map_plan_create(const vdx_fft_desc* desc, const char* hooks_source, vdx_
               ") vdx_mapped(vdx::FftArgs a, vdx::MapArgs m) {\n  vdx::mapped_body<vdx::FixPlan<" +
               std::to_string(g.args.pp.n) + ", " + std::to_string(g.args.pp.T) + ", vdx::RList<" + radices + ">, " +
               std::to_string(maxe) + ">, " + (g.strided ? "true" : "false") + ", " + (g.f64 ? "double" : "float") +
-              ", " + std::to_string(mode) + ", VdxHooks>(a, m);\n}\n";
+              ", " + std::to_string(mode) + ", VdxHooks, " + (total < (1ll << 32) ? "true" : "false") + ">(a, m);\n}\n";
   rc = compile(p->source, g.dev, &p->mod);
   if (rc != VDX_OK) {
     delete p;
