@@ -91,37 +91,103 @@ __device__ __forceinline__ T block_reduce(T v, T* sh) {
   return v;
 }
 
-constexpr int kThreads = 512;
+// Stage 1: part p of row b covers elements [p*chunk, min(n, (p+1)*chunk)) and is
+// folded by W warps, about 64 elements per thread: a CTA of eight warps holds
+// 8 / W parts.  (One 512-thread CTA per part spent 16 instructions per element
+// on 4096-element parts, most of them on the block's fold: 1024 x 65536 floats
+// took 54.9 us, 46.3 us this way; 39.5 us is the copy rate.)  A thread takes
+// four neighbouring elements per step, in 16-byte loads where the part starts
+// on such a boundary and in single loads of the same elements otherwise, and
+// the fold's order depends on n alone, so results do too.
+constexpr int kWarps = 8;
+constexpr int kVec = 4;
 
-// stage 1: grid (nparts, batch); CTA p of row b covers elements
-// [p*chunk, min(n, (p+1)*chunk)) with a block-stride loop.
-template <class In, class T, int OP, int MAP>
-__global__ void __launch_bounds__(kThreads) k_reduce_partial(const In* __restrict__ in, long long n, long long chunk,
-                                                             T* __restrict__ part, int nparts) {
-  __shared__ T sh[32];
-  const long long b = blockIdx.y;
-  const In* row = in + b * n;
-  const long long lo = (long long)blockIdx.x * chunk;
-  long long hi = lo + chunk;
-  if (hi > n) hi = n;
-  T a0 = identity<T, OP>(), a1 = a0, a2 = a0, a3 = a0;
-  long long i = lo + threadIdx.x;
-  for (; i + 3 * kThreads < hi; i += 4 * kThreads) {
-    const In x0 = row[i], x1 = row[i + kThreads], x2 = row[i + 2 * kThreads], x3 = row[i + 3 * kThreads];
-    a0 = combine<T, OP>(a0, apply_map<In, T, MAP>(x0));
-    a1 = combine<T, OP>(a1, apply_map<In, T, MAP>(x1));
-    a2 = combine<T, OP>(a2, apply_map<In, T, MAP>(x2));
-    a3 = combine<T, OP>(a3, apply_map<In, T, MAP>(x3));
-  }
-  for (; i < hi; i += kThreads) a0 = combine<T, OP>(a0, apply_map<In, T, MAP>(row[i]));
-  T acc = combine<T, OP>(combine<T, OP>(a0, a1), combine<T, OP>(a2, a3));
-  acc = block_reduce<T, OP>(acc, sh);
-  if (threadIdx.x == 0) part[b * nparts + blockIdx.x] = acc;
+inline int part_warps(long long chunk) {
+  int w = 1;
+  while (w < kWarps && chunk > 64ll * 32 * w) w <<= 1;
+  return w;
 }
 
-// stage 2: one CTA per row folds nparts partials
+template <class In>
+struct alignas(sizeof(In) * kVec <= 16 ? sizeof(In) * kVec : 16) Pack {
+  In v[kVec];
+};
+
 template <class T, int OP>
-__global__ void __launch_bounds__(kThreads) k_reduce_final(const T* __restrict__ part, int nparts, T* __restrict__ out) {
+__device__ __forceinline__ T warp_reduce(T v) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v = combine<T, OP>(v, shfl_down(v, d));
+  return v;
+}
+
+template <class In, class T, int OP, int MAP>
+__global__ void __launch_bounds__(32 * kWarps) k_reduce_partial(const In* __restrict__ in, long long n, long long chunk,
+                                                                T* __restrict__ part, int nparts, int W) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int TH = 32 * W;  // threads of a part, a power of two
+  __shared__ T sh[kWarps];
+  const int g = threadIdx.x / TH, t = threadIdx.x & (TH - 1);
+  const long long b = blockIdx.y;
+  const int p = blockIdx.x * (kWarps / W) + g;
+  T a[kVec];
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) a[i] = identity<T, OP>();
+  const In* row = in + b * n;
+  const long long lo = (long long)p * chunk;
+  long long hi = lo + chunk;
+  if (hi > n) hi = n;
+  if (p < nparts) {
+    const In* q = row + lo;
+    const long long full = hi > lo ? (hi - lo) / (kVec * TH) : 0;  // whole steps of the part's threads
+    if (reinterpret_cast<unsigned long long>(q) % alignof(Pack<In>) == 0) {
+      const Pack<In>* v = reinterpret_cast<const Pack<In>*>(q) + t;
+#pragma unroll 4
+      for (long long s = 0; s < full; ++s) {
+        const Pack<In> x = v[s * TH];
+#pragma unroll
+        for (int i = 0; i < kVec; ++i) a[i] = combine<T, OP>(a[i], apply_map<In, T, MAP>(x.v[i]));
+      }
+    } else {
+#pragma unroll 4
+      for (long long s = 0; s < full; ++s) {
+        In x[kVec];
+#pragma unroll
+        for (int i = 0; i < kVec; ++i) x[i] = q[(s * TH + t) * kVec + i];
+#pragma unroll
+        for (int i = 0; i < kVec; ++i) a[i] = combine<T, OP>(a[i], apply_map<In, T, MAP>(x[i]));
+      }
+    }
+    for (long long e = lo + full * kVec * TH + t; e < hi; e += TH)
+      a[0] = combine<T, OP>(a[0], apply_map<In, T, MAP>(row[e]));
+  }
+  T acc = combine<T, OP>(combine<T, OP>(a[0], a[1]), combine<T, OP>(a[2], a[3]));
+  acc = warp_reduce<T, OP>(acc);
+  if (W > 1) {
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) sh[w] = acc;
+    __syncthreads();
+    if (t == 0)
+      for (int i = 1; i < W; ++i) acc = combine<T, OP>(acc, sh[w + i]);
+  }
+  if (t == 0 && p < nparts) part[b * nparts + p] = acc;
+}
+
+// Stage 2 folds the partials of a row in a fixed order: one warp per row for
+// up to 32 partials, else one CTA per row.  It is launched to start while
+// stage 1 drains and waits for stage 1's partials here.
+constexpr int kThreads = 512;
+template <class T, int OP>
+__global__ void __launch_bounds__(kThreads) k_reduce_final(const T* __restrict__ part, int nparts, long long rows,
+                                                           T* __restrict__ out) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (nparts <= 32) {
+    const long long b = (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    T acc = b < rows && lane < nparts ? part[b * nparts + lane] : identity<T, OP>();
+    acc = warp_reduce<T, OP>(acc);
+    if (lane == 0 && b < rows) out[b] = acc;
+    return;
+  }
   __shared__ T sh[32];
   const long long b = blockIdx.x;
   T acc = identity<T, OP>();
@@ -132,15 +198,21 @@ __global__ void __launch_bounds__(kThreads) k_reduce_final(const T* __restrict__
 
 template <class In, class T, int OP, int MAP>
 cudaError_t run(const void* in, long long n, long long batch, void* out, void* partials, int nparts, cudaStream_t s) {
-  const long long chunk = (n + nparts - 1) / nparts;
-  dim3 g1((unsigned)nparts, (unsigned)batch);
-  k_reduce_partial<In, T, OP, MAP><<<g1, kThreads, 0, s>>>(reinterpret_cast<const In*>(in), n, chunk,
-                                                          reinterpret_cast<T*>(partials), nparts);
-  cudaError_t e = cudaGetLastError();
+  // parts start on 16-byte steps of the row
+  const long long chunk = ((n + nparts - 1) / nparts + 3) & ~3ll;
+  const int W = part_warps(chunk), G = kWarps / W;
+  const Launch l1{dim3((unsigned)((nparts + G - 1) / G), (unsigned)batch), dim3(32 * kWarps), 0, s};
+  const In* src = reinterpret_cast<const In*>(in);
+  T* part = reinterpret_cast<T*>(partials);
+  cudaError_t e = enqueue(k_reduce_partial<In, T, OP, MAP>, l1, src, n, chunk, part, nparts, W);
   if (e != cudaSuccess) return e;
-  k_reduce_final<T, OP><<<(unsigned)batch, kThreads, 0, s>>>(reinterpret_cast<const T*>(partials), nparts,
-                                                             reinterpret_cast<T*>(out));
-  return cudaGetLastError();
+  Launch l2{dim3((unsigned)batch), dim3(kThreads), 0, s};
+  if (nparts <= 32) {
+    l2.block = dim3(batch == 1 ? 32 : 128);
+    l2.grid = dim3((unsigned)((batch + l2.block.x / 32 - 1) / (l2.block.x / 32)));
+  }
+  const T* cpart = part;
+  return enqueue_pdl(k_reduce_final<T, OP>, l2, cpart, nparts, batch, reinterpret_cast<T*>(out));
 }
 
 template <class In, class T, int OP>
