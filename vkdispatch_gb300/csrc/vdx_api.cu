@@ -1025,10 +1025,17 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
                       std::getenv("VDX_NO_FIXED") == nullptr;
   const bool is_conv = d.kind == VDX_KIND_CONV;
   int pmaxe = (tune.maxe == 8 || tune.maxe == 32) ? tune.maxe : 16;
-  // default for strided complex64 convolutions of 512 or 1024 points: the
-  // two-pass radix-32 plan (64 x 512 x 257 along axis 1: 58.0 us against
-  // 70.3 us for radix 16 x 16 x 2, each launch alone from a cold L2)
-  if (tune.maxe == 0 && is_conv && inner > 1 && canpts && has_fixedpts_c64(n, 32, true, true)) pmaxe = 32;
+  // the two-pass radix-32 plan is the default of strided complex64 transforms
+  // and convolutions of 512 or 1024 points and of 512-point convolutions along
+  // rows (each launch alone from a cold L2, radix-16 plan -> radix-32 plan:
+  // 64 x 512 x 512 C2C along axis 1 56.0 -> 53.3 us, 16 x 1024 x 1024 68.3 ->
+  // 60.5, convolutions 64 x 512 x 257 59.9 -> 49.1, 16 x 1024 x 513 86.9 ->
+  // 82.1, 32768 x 512 rows 89.9 -> 72.5); rows of C2C are indifferent (85.9 ->
+  // 85.0, 84.5 -> 86.5) and 1024-point convolutions along rows lose (96.2 ->
+  // 118.6)
+  if (tune.maxe == 0 && !real && canpts && has_fixedpts_c64(n, 32, is_conv, inner > 1) &&
+      (inner > 1 || (is_conv && n == 512)))
+    pmaxe = 32;
   if (const char* e = std::getenv("VDX_POINTS_PER_THREAD")) {
     const int v = std::atoi(e);
     if (v == 16) pmaxe = 16;
