@@ -1038,61 +1038,75 @@ __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 3
              GlobalOut<S, Re>(a, pl));
 }
 
-// Strided fused convolution for CTAs of at most 256 threads, complex64.  The
-// launch bound allows 128 registers per thread (80 for plans of 8 points
-// per thread).  Plans of up to 16 points per thread load the kernel
-// spectrum into registers right after issuing the signal loads, so its HBM
-// latency overlaps the forward passes instead of following them; with 32
-// points per thread the registers are full and it is loaded after the
-// forward FFT.  The kernel spectrum is read once, with evict-first loads.
-template <class Plan, class S, class Re, int KOP>
+// Fused convolution for CTAs of at most 256 threads, complex64 compile-time
+// plans.  The launch bound allows 128 registers per thread (80 for plans of 8
+// points per thread).  Plans of up to 16 points per thread load the kernel
+// spectrum (and SPEC 2's spec_aux) into registers right after issuing the
+// signal loads, so its HBM latency overlaps the forward passes instead of
+// following them (rows: 65536 x 256 points 82.2 -> 67.0 us, 16384 x 1024 98.5 ->
+// 77.0, 8192 x 2048 112.1 -> 85.3); with 32 points per thread the registers are
+// full and it is loaded after the forward FFT.  The kernel spectrum is read
+// once, with evict-first loads.
+template <class Plan, bool STRIDED, class S, class Re, int KOP, int SPEC = 0>
 __global__ void __launch_bounds__(256, Plan::MAXE <= 8 ? 3 : 2) k_conv_pf(FftArgs a) {
   pdl_enter();
   const Plan P(a.pp);
-  constexpr int MAXE = Plan::MAXE;
-  const Place<true> pl(a, P.T());
+  constexpr int MAXE = Plan::MAXE, RR = Plan::kLast;
+  const Place<STRIDED> pl(a, P.T());
   Cx<Re>* sm = smem_base<Re>();
   const Cx<Re>* tw = reinterpret_cast<const Cx<Re>*>(a.tw);
   const Cx<Re>* twr = reinterpret_cast<const Cx<Re>*>(a.twr);
   const S* ker = reinterpret_cast<const S*>(a.ker) + pl.ker0();
   P.assume_t(pl.t);
-  const int n = P.n();
+  const int n = P.n(), nb = n / RR;
   const bool kvalid = pl.tile_full || pl.valid;
+  const long long step = nb * pl.ps;
   constexpr bool PF = MAXE <= 16;
   Cx<Re> v[MAXE];
   gather_input<Plan, S, Re>(P, pl, a, v);
-  Cx<Re> kr[PF ? MAXE : 1];
-  if constexpr (PF) P.template last<false>([&](auto rc) {
-    constexpr int RR = decltype(rc)::value;
-    constexpr int B = MAXE / RR;
-    const int nb = n / RR;
-#pragma unroll
-    for (int b = 0; b < B; ++b) {
-      const int j = pl.t + b * P.T();
+  Cx<Re> kr[PF ? MAXE : 1], ar[PF && SPEC == 2 ? MAXE : 1];
+  if constexpr (PF) {
+    Plan::template each<RR>(pl.t, [&](auto b, int j) {
       const S* q = ker + j * pl.ps;
-      const long long step = nb * pl.ps;
 #pragma unroll
-      for (int r = 0; r < RR; ++r, q += step)
-        kr[b * RR + r] = (j < nb && kvalid) ? ld_once<S, Re>(q) : mk<Re>(Re(0), Re(0));
+      for (int r = 0; r < RR; ++r, q += step) kr[b * RR + r] = kvalid ? ld_once<S, Re>(q) : mk<Re>(Re(0), Re(0));
+    });
+    if constexpr (SPEC == 2) {
+      Plan::template each<RR>(pl.t, [&](auto b, int j) {
+        const S* q = reinterpret_cast<const S*>(a.spec_aux) + pl.out0() + j * pl.ps;
+#pragma unroll
+        for (int r = 0; r < RR; ++r, q += step) ar[b * RR + r] = kvalid ? ld_once<S, Re>(q) : mk<Re>(Re(0), Re(0));
+      });
     }
-  });
+  }
   P.template run<false, false, true>(v, pl, sm, tw);
-  P.template last<false>([&](auto rc) {
-    constexpr int RR = decltype(rc)::value;
-    constexpr int B = MAXE / RR;
-    const int nb = n / RR;
+  if constexpr (SPEC != 0) {
+    Plan::template each<RR>(pl.t, [&](auto b, int j) {
+      if (!kvalid) return;
+      S* q = reinterpret_cast<S*>(a.spec_out) + pl.out0() + j * pl.ps;
+      const S* x = reinterpret_cast<const S*>(a.spec_aux) + pl.out0() + j * pl.ps;
 #pragma unroll
-    for (int b = 0; b < B; ++b) {
-      const int j = pl.t + b * P.T();
-      const S* q = ker + j * pl.ps;
-      const long long step = nb * pl.ps;
-#pragma unroll
-      for (int r = 0; r < RR; ++r, q += step) {
-        Cx<Re> k;
-        if constexpr (PF) k = kr[b * RR + r];
-        else k = (j < nb && kvalid) ? ld_once<S, Re>(q) : mk<Re>(Re(0), Re(0));
-        v[b * RR + r] = KOP == 0 ? cmulc(v[b * RR + r], k) : cmul(v[b * RR + r], k);
+      for (int r = 0; r < RR; ++r, q += step, x += step) {
+        const Cx<Re> f = v[b * RR + r];
+        if constexpr (SPEC == 1) {
+          Conv<S, Re>::st(q, f);
+        } else {
+          Cx<Re> g;
+          if constexpr (PF) g = ar[b * RR + r];
+          else g = Conv<S, Re>::ld(x);
+          Conv<S, Re>::st(q, scale(cmulc(g, f), Re(a.spec_scale)));
+        }
       }
+    });
+  }
+  Plan::template each<RR>(pl.t, [&](auto b, int j) {
+    const S* q = ker + j * pl.ps;
+#pragma unroll
+    for (int r = 0; r < RR; ++r, q += step) {
+      Cx<Re> k;
+      if constexpr (PF) k = kr[b * RR + r];
+      else k = kvalid ? ld_once<S, Re>(q) : mk<Re>(Re(0), Re(0));
+      v[b * RR + r] = KOP == 0 ? cmulc(v[b * RR + r], k) : cmul(v[b * RR + r], k);
     }
   });
   P.template run<true, true>(v, pl, sm, twr);

@@ -7,8 +7,8 @@
 
 namespace vdx {
 
-// Strided compile-time convolutions of <= 256-thread CTAs load the kernel
-// spectrum before the forward FFT (k_conv_pf) unless VDX_CONV_PREFETCH=0.
+// Compile-time convolutions of <= 256-thread CTAs load the kernel spectrum
+// before the forward FFT (k_conv_pf) unless VDX_CONV_PREFETCH=0.
 inline bool conv_prefetch() {
   static const bool on = [] {
     const char* e = std::getenv("VDX_CONV_PREFETCH");
@@ -43,8 +43,15 @@ cudaError_t launch_c2c(const FftArgs& a, const Launch& l, bool strided, int vari
 template <class Plan, int KOP, bool STRIDED, class S, class Re>
 cudaError_t launch_conv_layout(const FftArgs& a, const Launch& l, int variant) {
   constexpr bool C64 = std::is_same<S, Cx<float>>::value;
-  if constexpr (C64 && STRIDED && IsFixPlan<Plan>::value) {
-    if (variant == 0 && l.block.x <= 256 && conv_prefetch()) return enqueue_pdl(k_conv_pf<Plan, S, Re, KOP>, l, a);
+  if constexpr (C64 && IsFixPlan<Plan>::value) {
+    if (l.block.x <= 256 && conv_prefetch()) {
+      if (variant == 0) return enqueue_pdl(k_conv_pf<Plan, STRIDED, S, Re, KOP>, l, a);
+      if constexpr (KOP == 0) {
+        if (variant == 1) return enqueue_pdl(k_conv_pf<Plan, STRIDED, S, Re, 0, 1>, l, a);
+      } else {
+        if (variant == 2) return enqueue_pdl(k_conv_pf<Plan, STRIDED, S, Re, 1, 2>, l, a);
+      }
+    }
   }
   if constexpr (C64 && KOP == 0) {
     if (variant == 1) return enqueue_pdl(k_conv<Plan, STRIDED, S, S, Re, 0, 1>, l, a);
