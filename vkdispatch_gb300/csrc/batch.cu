@@ -59,7 +59,7 @@ struct UnitPlan {
   const Cx<float>* tw;  // stage-ordered twiddles of this pass plan
 };
 
-struct WorkUnit {
+struct alignas(16) WorkUnit {
   PassPlan pp;                  // the unit's pass plan (a copy, so one table read fetches everything)
   const Cx<float>* tw;          // stage-ordered twiddles of the unit's pass plan
   long long src, dst;           // element offset of point 0 of slot 0 (data or workspace)
@@ -120,7 +120,7 @@ struct UnitIn {
 };
 // Column units multiply by the four-step twiddles W_L^{n2 k1} of the thread's
 // column n2, which are laid out like the column's points.
-// The sink's fields are read from the unit table when the last pass stores, so
+// The sink's fields are read from the descriptor when the last pass stores, so
 // they hold no registers during the passes.
 template <bool INV>
 struct UnitOut {
@@ -161,8 +161,7 @@ template <bool INV>
 __device__ __forceinline__ void run_unit(const BatchArgs& a, const WorkUnit* __restrict__ pu, int kind,
                                          Cx<float>* sm) {
   constexpr int MAXE = 16;
-  // fields are read from the (L1-cached, CTA-uniform) unit table: read-only
-  // global loads the compiler may repeat instead of holding them in registers
+  // fields are read from shared memory where they are needed rather than held
   const WorkUnit& wu = *pu;
   const PassPlan& pp = wu.pp;
   const int n = pp.n, T = pp.T, M = pp.M;
@@ -227,7 +226,21 @@ __device__ __forceinline__ void run_unit(const BatchArgs& a, const WorkUnit* __r
 // round trip to L2 lies between two units.  A CTA may hold two claimed
 // units, but a claimed UK_COLS unit only ever follows another UK_COLS unit
 // of the same CTA, which does not wait, so every claimed UK_COLS unit runs.
-constexpr int kUnitLines = int((sizeof(WorkUnit) + 127) / 128) + 1;  // 128-byte lines a descriptor touches
+//
+// Descriptors are read from shared memory: the next unit's is copied there
+// (cp.async) while the current unit runs.  In global memory the lines a unit's
+// passes come back to are pushed out of L1 by the tile streaming through it,
+// and every pass starts with a trip to L2 (1024 items of 2^26 points, forward and
+// inverse: 1262 us from global memory, 1156 us from shared memory).
+constexpr int kUnitWords = int(sizeof(WorkUnit) / 16);
+
+__device__ __forceinline__ void fetch_unit(WorkUnit* dst, const WorkUnit* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst) + 16 * threadIdx.x;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d),
+               "l"(reinterpret_cast<const char*>(src) + 16 * threadIdx.x)
+               : "memory");
+}
+__device__ __forceinline__ void fetch_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <bool INV, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) k_batch(BatchArgs a) {
@@ -235,6 +248,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_batch(BatchArgs a) {
   // that one barrier per unit separates their reads from the next writes
   __shared__ int s_cur[2], s_next[2];
   __shared__ int s_ok;
+  __shared__ WorkUnit s_unit[2];  // current and next, by iteration parity
   Cx<float>* sm = smem_base<float>();
   const int tid = threadIdx.x;
   int claim = 0;  // thread 0: the ticket two units ahead
@@ -244,15 +258,15 @@ __global__ void __launch_bounds__(THREADS, MINB) k_batch(BatchArgs a) {
     claim = s_next[0] < a.nunits ? (int)atomicAdd(a.ticket, 1u) : a.nunits;
   }
   __syncthreads();
+  if (tid < kUnitWords && s_cur[0] < a.nunits) fetch_unit(&s_unit[0], &a.units[s_cur[0]]);
+  fetch_done();
+  __syncthreads();
   for (int par = 0;; par ^= 1) {
     const int u = s_cur[par];
     if (u >= a.nunits) return;
     const int un = s_next[par];
-    if (tid < kUnitLines && un < a.nunits) {
-      const char* line = reinterpret_cast<const char*>(&a.units[un]) + 128 * tid;
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(line));
-    }
-    const WorkUnit* pu = &a.units[u];
+    if (tid < kUnitWords && un < a.nunits) fetch_unit(&s_unit[par ^ 1], &a.units[un]);
+    const WorkUnit* pu = &s_unit[par];
     const WorkUnit& wu = *pu;
     const int kind = wu.kind;
     bool run = true;
@@ -293,6 +307,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_batch(BatchArgs a) {
       s_next[par ^ 1] = claim;
       if (claim < a.nunits) claim = (int)atomicAdd(a.ticket, 1u);
     }
+    fetch_done();  // the next descriptor has landed; the barrier shows it to every thread
     __syncthreads();
   }
 }
