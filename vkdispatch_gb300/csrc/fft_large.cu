@@ -22,6 +22,8 @@
 
 namespace vdx {
 
+int fourstep_pitch(const PassPlan& pp) { return fs_pitch(pp.M, pp.T); }
+
 cudaError_t launch_fourstep_pass(const FsArgs& a, const Launch& l, int store, bool inv, int mode) {
   switch (store) {
     case ST_C64: return launch_fs_c64(a, l, inv, mode);

@@ -62,8 +62,13 @@ struct FsOut {
 
 // MODE 0: plain store (pass B).  MODE 1: four-step twiddle, then a store
 // whose columns are unit-stride (strided axes).  MODE 2: four-step twiddle,
-// then a transposed store through shared memory so that each column's points
-// land contiguously (out_ps == 1; contiguous axes).
+// then a store in which each column's points land contiguously (out_ps == 1;
+// contiguous axes).  Compile-time plans transpose in the exchange they make
+// anyway: the first pass runs with neighbouring columns in neighbouring lanes,
+// as the loads want, and the last with neighbouring points, as the stores want
+// (16384^2 bf16 along rows: 1047 -> 917 us for both passes; 384 x 65536: 145.5 ->
+// 131.3 us).  Runtime plans transpose through shared memory
+// after the last pass.
 template <bool INV, class S, int MODE, class Plan, class In>
 __device__ __forceinline__ void fs_transform(const Plan& P, const FsPlace& pl, const FsArgs& a, const In& in, S* out,
                                              const Cx<float>* twl, int col, bool valid, Cx<float>* sm) {
@@ -71,11 +76,51 @@ __device__ __forceinline__ void fs_transform(const Plan& P, const FsPlace& pl, c
   if constexpr (MODE == 2) {
     // odd row pitch n + 1: the column-major writes spread over the banks
     P.template transform<INV, false, true>(
-        pl, sm, tw, in, FsOut<Cx<float>, INV, true>{sm + pl.m * (P.n() + 1), 1, twl, a.tw_ld, a.scale, true});
+        pl, sm, tw, in, FsOut<Cx<float>, INV, true>{sm + pl.m * (P.n() + 1), 1, twl, a.tw_p, a.scale, true});
   } else {
     P.template transform<INV, false, false>(
-        pl, sm, tw, in, FsOut<S, INV, MODE == 1>{out + col, a.out_ps, twl, a.tw_ld, a.scale, valid});
+        pl, sm, tw, in, FsOut<S, INV, MODE == 1>{out + col, a.out_ps, twl, a.tw_p, a.scale, valid});
   }
+}
+
+// slots between neighbouring points of a transposing exchange: columns in
+// lanes on one side and T threads' points on the other without bank conflicts
+__host__ __device__ constexpr int fs_pitch(int M, int T) { return T <= 16 ? M + 16 / T : M + 1; }
+
+// MODE 2 of a two-pass compile-time plan
+template <bool INV, class S, class Plan, class In>
+__device__ __forceinline__ void fs_transpose(const Plan& P, const FsPlace& pl, const FsArgs& a, const In& in, S* out,
+                                             int tile, Cx<float>* sm) {
+  constexpr int R0 = Plan::kFirst, R1 = Plan::kLast, N = R0 * R1, T = Plan::T(), MAXE = Plan::MAXE;
+  static_assert(Plan::n() == N, "two passes");
+  const int pitch = fs_pitch(pl.M, T);
+  Cx<float> v[MAXE];
+  Plan::template each<R0>(pl.t, [&](auto b, int j) {
+    in.template load<R0>(&v[b * R0], j, N / R0);
+    Dft<R0, INV, float>::run(&v[b * R0]);
+    Cx<float>* q = sm + j * R0 * pitch + pl.m;
+#pragma unroll
+    for (int r = 0; r < R0; ++r, q += pitch) *q = v[b * R0 + r];
+  });
+  __syncthreads();
+  const int t = threadIdx.x % T, m = threadIdx.x / T;
+  const int c = tile * pl.M + m;
+  if (c >= a.ncols) return;
+  const Cx<float>* tw = reinterpret_cast<const Cx<float>*>(a.tw);
+  const Cx<float>* w = reinterpret_cast<const Cx<float>*>(a.twl) + c * a.tw_b;
+  S* dst = out + c * a.out_cs;
+  Plan::template each<R1>(t, [&](auto b, int j) {
+    const Cx<float>* q = sm + j * pitch + m;
+#pragma unroll
+    for (int r = 0; r < R1; ++r, q += R0 * pitch) v[b * R1 + r] = *q;
+    twiddled_dft<R1, INV>(&v[b * R1], j, R0, tw);
+#pragma unroll
+    for (int r = 0; r < R1; ++r) {
+      const int pos = j + r * R0;
+      const Cx<float> f = ldg(w + pos * a.tw_p);
+      Conv<S, float>::st(dst + pos, scale(INV ? cmulc(v[b * R1 + r], f) : cmul(v[b * R1 + r], f), a.scale));
+    }
+  });
 }
 
 template <class Plan, bool INV, class S, int MODE>
@@ -99,11 +144,15 @@ __global__ void __launch_bounds__(512, 2) k_fs(FsArgs a) {
   // cross twiddles of column b0 < N0.  Columns past the last one of a partial
   // tile (col >= ncols) take b0 = 0: theirs would lie past the table
   const int b0 = a.tw_from_batch ? (int)br : (valid ? col : 0);
-  const Cx<Re>* twl = reinterpret_cast<const Cx<Re>*>(a.twl) + b0;
-  fs_transform<INV, S, MODE>(
-      P, pl, a, FsIn<S>{reinterpret_cast<const S*>(a.in) + bq * a.in_bs1 + br * a.in_bs2 + col, a.in_ps, valid}, out,
-      twl, col, valid, sm);
-  if constexpr (MODE == 2) {
+  const Cx<Re>* twl = reinterpret_cast<const Cx<Re>*>(a.twl) + b0 * a.tw_b;
+  const FsIn<S> in{reinterpret_cast<const S*>(a.in) + bq * a.in_bs1 + br * a.in_bs2 + col, a.in_ps, valid};
+  if constexpr (MODE == 2 && IsFixPlan<Plan>::value) {
+    fs_transpose<INV, S>(P, pl, a, in, out, tile, sm);
+    return;
+  } else {
+    fs_transform<INV, S, MODE>(P, pl, a, in, out, twl, col, valid, sm);
+  }
+  if constexpr (MODE == 2 && !IsFixPlan<Plan>::value) {
     __syncthreads();
     const long long ocs = a.out_cs;
     const int total = n * M, ld = n + 1;
@@ -130,7 +179,7 @@ cudaError_t launch_mode(const FsArgs& a, const Launch& l, bool inv, int mode) {
 
 template <class S>
 cudaError_t launch_any(const FsArgs& a, const Launch& l, bool inv, int mode) {
-  const int n = a.pp.n, T = a.pp.T;
+  const int n = a.pp.n, T = a.pp.T;  // the lengths below: fourstep_fixed()
   if (n == 128 && T == 8) return launch_mode<FixPlan<128, 8, RList<16, 8>>, S>(a, l, inv, mode);
   if (n == 256 && T == 16) return launch_mode<FixPlan<256, 16, RList<16, 16>>, S>(a, l, inv, mode);
   if (n == 64 && T == 4) return launch_mode<FixPlan<64, 4, RList<16, 4>>, S>(a, l, inv, mode);

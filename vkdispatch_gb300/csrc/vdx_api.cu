@@ -633,6 +633,10 @@ int plan_fourstep(vdx_plan* p, long long inner, long long outer, int smem_optin)
   p->blockB = dim3(ppB.T * ppB.M);
   p->smemA = size_t(std::max(N1 * ppA.M, (N1 + 1) * ppA.M)) * 8;
   p->smemB = size_t(N0) * ppB.M * 8;
+  // the transposed stores of compile-time plans run along a column's points,
+  // the other stores across columns: the cross twiddles are laid out to match
+  const bool by_point = !strided && !p->tensor_core && fourstep_fixed(ppA);
+  if (by_point) p->smemA = size_t(N1) * fourstep_pitch(ppA) * 8;
   // the tensor-core passes read natural tables, the butterfly passes stage-ordered ones
   auto short_table = [&](const PassPlan& pp, const void** out) {
     void** o = const_cast<void**>(out);
@@ -643,8 +647,10 @@ int plan_fourstep(vdx_plan* p, long long inner, long long outer, int smem_optin)
   if (rc == VDX_OK) rc = short_table(ppB, &p->fsB.tw);
   if (rc == VDX_OK)
     rc = p->tensor_core ? get_table(p->dev, N, N, false, const_cast<void**>(&p->fsA.twl))
-                        : build_cross_table(p->dev, N1, N0, const_cast<void**>(&p->fsA.twl));
-  p->fsA.tw_ld = N0;
+                        : build_cross_table(p->dev, by_point ? N0 : N1, by_point ? N1 : N0,
+                                            const_cast<void**>(&p->fsA.twl));
+  p->fsA.tw_b = by_point ? N1 : 1;
+  p->fsA.tw_p = by_point ? 1 : N0;
   if (rc != VDX_OK) return rc;
   p->fsA.scale = 1.f;
   p->fsB.scale = float(p->args.scale);

@@ -78,8 +78,8 @@ struct FsArgs {
   const void* in;
   void* out;
   const void* tw;   // stage-ordered twiddles of the short transform (tensor-core passes: W_n^k)
-  const void* twl;  // pass A: cross twiddles W_N^{b0 k1} at k1 * tw_ld + b0 (tensor-core passes: W_N^k)
-  int tw_ld;
+  const void* twl;  // pass A: cross twiddles W_N^{b0 k1} at b0 * tw_b + k1 * tw_p (tensor-core passes: W_N^k)
+  int tw_b, tw_p;
   long long split;
   long long in_bs1, in_bs2, out_bs1, out_bs2;
   long long in_ps, out_ps, out_cs;
@@ -89,6 +89,12 @@ struct FsArgs {
   long long nbatch;   // batches of this launch (grid = nbatch * col_tiles)
 };
 // mode 0: plain store; 1: twiddle, unit-stride columns; 2: twiddle, transposed store (out_ps == 1).
+// Whether a short length runs on a compile-time plan, whose transposed stores
+// read the cross twiddles along k1, and the exchange pitch of those stores.
+inline bool fourstep_fixed(const PassPlan& pp) {
+  return (pp.n == 128 && pp.T == 8) || (pp.n == 256 && pp.T == 16) || (pp.n == 64 && pp.T == 4);
+}
+int fourstep_pitch(const PassPlan& pp);
 cudaError_t launch_fourstep_pass(const FsArgs& a, const Launch& l, int store, bool inv, int mode);
 // The same pass with the 128-point short transforms on the tensor cores
 // (fft_tc.cu); a.pp.n must be 128 and a.pp.M 16 or 32.  bmat = the DFT
