@@ -49,9 +49,9 @@ def test_real_rows(n):
 
 
 @pytest.mark.parametrize("storage,tol", [(vd.complex32, 2.5e-3), (vd.complexbf16, 1.6e-2)])
-@pytest.mark.parametrize("n", [16, 48, 64, 150, 512, 1500, 2048])
+@pytest.mark.parametrize("n", [16, 32, 48, 64, 128, 150, 256, 512, 1024, 1500, 2048, 4096])
 def test_half_storage(n, storage, tol):
-    """16-bit storage runs powers of two on the runtime passes, with padded rows."""
+    """16-bit storage: compile-time plans of powers of two up to 4096 points, runtime passes besides."""
     rng = np.random.default_rng(n)
     for shape, axis in (((5, n), 1), ((2, n, 9), 1)):
         x = crandn(rng, shape) * 0.25
@@ -60,6 +60,9 @@ def test_half_storage(n, storage, tol):
         q = b.read(0).astype(np.complex128)
         vd.fft.fft(b, axis=axis)
         assert rel_l2(b.read(0), np.fft.fft(q, axis=axis)) <= tol
+        q = b.read(0).astype(np.complex128)
+        vd.fft.ifft(b, axis=axis)
+        assert rel_l2(b.read(0), np.fft.ifft(q, axis=axis)) <= tol
 
 
 def test_uneven_batch_of_composite_radices():

@@ -25,6 +25,16 @@ cudaError_t launch_fixed_c64_any(int n, const FftArgs& a, const Launch& l, int o
   }
 }
 
+bool has_fixed_half(int n) { return n >= 16 && n <= 4096 && (n & (n - 1)) == 0; }
+
+cudaError_t launch_fixed_half(int store, int n, const FftArgs& a, const Launch& l, int op, bool strided) {
+  if (store == ST_C32)
+    return n <= 256 ? launch_fixed_c32_small(n, a, l, op, strided) : launch_fixed_c32_large(n, a, l, op, strided);
+  if (store == ST_BF16)
+    return n <= 256 ? launch_fixed_bf16_small(n, a, l, op, strided) : launch_fixed_bf16_large(n, a, l, op, strided);
+  return cudaErrorInvalidValue;
+}
+
 bool has_fixedpts_c64(int n, int pts, bool conv, bool strided) {
   if (pts == 8) return conv && strided && n == 512;
   return pts == 32 && (n == 512 || n == 1024);

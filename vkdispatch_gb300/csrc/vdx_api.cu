@@ -358,6 +358,7 @@ struct vdx_plan {
   int store;
   int N;  // axis length (real length for R2C/C2R)
   bool fixed;  // compile-time specialised kernels (complex64, power-of-two n)
+  bool fixed_half = false;  // the same for C2C of 16-bit storage
   FftArgs args;
   Launch launch;
   std::vector<int> radices;
@@ -1223,6 +1224,8 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
                   (pmaxe == 32 || (p->op == OP_CONV && strided)))
                      ? pmaxe
                      : 0;
+  p->fixed_half = (st == ST_C32 || st == ST_BF16) && d.kind == VDX_KIND_C2C && has_fixed_half(n) && T == n / 16 &&
+                  std::getenv("VDX_NO_FIXED") == nullptr && tune.order == 0 && tune.fixed != 0;
   if (pmaxe != 16 && !p->fixed_pts) {
     delete p;
     return fail(VDX_ERR_UNSUPPORTED, "no compile-time plan of 8 points per thread for this convolution");
@@ -1609,7 +1612,7 @@ int vdx_fft_plan_describe(const vdx_plan* p, char* buf, size_t n) {
                 "\"transforms_per_cta\": %d, \"strided\": %s, \"fixed\": %s, \"grid\": %u, \"block\": %u, "
                 "\"smem\": %zu, \"autotuned\": %s, \"tune\": [%d, %d, %d, %d, %d], \"tune_candidates\": %d}",
                 ops[p->op], p->N, p->args.pp.n, r.c_str(), p->args.pp.T, p->args.pp.M, p->strided ? "true" : "false",
-                (p->fixed || p->fixed_pts) ? "true" : "false", p->launch.grid.x, p->launch.block.x, p->launch.smem,
+                (p->fixed || p->fixed_half || p->fixed_pts) ? "true" : "false", p->launch.grid.x, p->launch.block.x, p->launch.smem,
                 p->tuned ? "true" : "false", p->tune.width, p->tune.order, p->tune.fixed, p->tune.fourstep,
                 p->tune.maxe, p->tuned_candidates);
   return VDX_OK;
@@ -1739,6 +1742,11 @@ int exec_plan(const vdx_plan* p, const void* in, void* out, const void* kernel, 
   }
   if (p->fixed) {
     e = launch_fixed_c64_any(p->args.pp.n, a, l, p->op, p->strided, p->d.kernel_op, variant);
+    if (e != cudaSuccess) return cuda_fail(e, "FFT launch");
+    return VDX_OK;
+  }
+  if (p->fixed_half && variant == 0) {
+    e = launch_fixed_half(p->store, p->args.pp.n, a, l, p->op, p->strided);
     if (e != cudaSuccess) return cuda_fail(e, "FFT launch");
     return VDX_OK;
   }

@@ -167,6 +167,16 @@ cudaError_t launch_fixed_c64(const FftArgs& a, const Launch& l, int op, bool str
 bool has_fixed_c64(int n);
 cudaError_t launch_fixed_c64_any(int n, const FftArgs& a, const Launch& l, int op, bool strided, int kop,
                                  int variant);
+// C2C kernels of 16-bit storage on the same plans, n in [16, 4096]: their
+// bytes are half of complex64's, so they are bound by instructions, which the
+// runtime-radix kernels spend on addresses (32768 x 1024 bf16 points: 95.1 us
+// on the runtime passes, 67.8 us here; 256^3 fp16 along axis 0: 43.3 and 36.3)
+bool has_fixed_half(int n);
+cudaError_t launch_fixed_half(int store, int n, const FftArgs& a, const Launch& l, int op, bool strided);
+cudaError_t launch_fixed_c32_small(int n, const FftArgs& a, const Launch& l, int op, bool strided);
+cudaError_t launch_fixed_c32_large(int n, const FftArgs& a, const Launch& l, int op, bool strided);
+cudaError_t launch_fixed_bf16_small(int n, const FftArgs& a, const Launch& l, int op, bool strided);
+cudaError_t launch_fixed_bf16_large(int n, const FftArgs& a, const Launch& l, int op, bool strided);
 // complex64 kernels on the alternative compile-time plans: pts = 32 (two
 // passes: radix 32 x 16 for n = 512, 32 x 32 for n = 1024; n/32 threads per
 // transform) for every operation, and pts = 8 (radix-8 passes, n/8 threads)
