@@ -125,8 +125,10 @@ def _packed(shape_real, dtype):
 
 def _dense_rows(x: torch.Tensor) -> bool:
     """Whether a contiguous real tensor's rows can be read as complex elements
-    in place: even length, first element on a complex element's alignment."""
-    return x.numel() > 0 and x.shape[-1] % 2 == 0 and x.data_ptr() % (2 * x.element_size()) == 0
+    in place: even length, first element on a complex element's alignment, on
+    the device that the plan runs on."""
+    return (x.numel() > 0 and x.shape[-1] % 2 == 0 and x.data_ptr() % (2 * x.element_size()) == 0
+            and x.device.index == torch.cuda.current_device())
 
 
 def _rfft_raw(x: torch.Tensor) -> torch.Tensor:
@@ -150,7 +152,7 @@ def _rfft_raw(x: torch.Tensor) -> torch.Tensor:
 def _irfft_raw(h: torch.Tensor, n: int, scale_1n: bool) -> torch.Tensor:
     io, comp = _IO[h.dtype]
     shape = tuple(h.shape[:-1]) + (n,)
-    if n % 2 == 0 and h.numel() > 0 and h.shape[-1] == n // 2 + 1:
+    if n % 2 == 0 and h.numel() > 0 and h.shape[-1] == n // 2 + 1 and h.device.index == torch.cuda.current_device():
         h = _raw(h)
         y = torch.empty(shape, dtype=torch.float32 if h.dtype == torch.complex64 else torch.float64, device="cuda")
         P.get_plan(shape, len(shape) - 1, L.VDX_KIND_C2R, True, scale_1n, io, comp,

@@ -220,9 +220,9 @@ __device__ __forceinline__ void run_unit(const BatchArgs& a, const WorkUnit* __r
 // THREADS per CTA, MINB resident CTAs per SM (64 registers per thread).
 //
 // Claiming runs two units ahead: while a CTA works on unit u it already
-// knows the next unit, whose descriptor (pass plan included) is prefetched
-// into L1 at the start of u, and thread 0 holds the ticket of the one after,
-// whose atomic was issued a whole unit earlier.  No ticket or pass-plan
+// knows the next unit, whose descriptor (pass plan included) is on its way to
+// shared memory, and thread 0 holds the ticket of the one after, whose atomic
+// was issued a whole unit earlier.  No ticket or pass-plan
 // round trip to L2 lies between two units.  A CTA may hold two claimed
 // units, but a claimed UK_COLS unit only ever follows another UK_COLS unit
 // of the same CTA, which does not wait, so every claimed UK_COLS unit runs.
@@ -230,8 +230,8 @@ __device__ __forceinline__ void run_unit(const BatchArgs& a, const WorkUnit* __r
 // Descriptors are read from shared memory: the next unit's is copied there
 // (cp.async) while the current unit runs.  In global memory the lines a unit's
 // passes come back to are pushed out of L1 by the tile streaming through it,
-// and every pass starts with a trip to L2 (1024 items of 2^26 points, forward and
-// inverse: 1262 us from global memory, 1156 us from shared memory).
+// and every pass starts with a trip to L2 (1024 items of 2^26 points, forward
+// and inverse: 1262 us from global memory, 1156 us from shared memory).
 constexpr int kUnitWords = int(sizeof(WorkUnit) / 16);
 
 __device__ __forceinline__ void fetch_unit(WorkUnit* dst, const WorkUnit* src) {

@@ -66,9 +66,9 @@ struct FsOut {
 // contiguous axes).  Compile-time plans transpose in the exchange they make
 // anyway: the first pass runs with neighbouring columns in neighbouring lanes,
 // as the loads want, and the last with neighbouring points, as the stores want
-// (16384^2 bf16 along rows: 1047 -> 917 us for both passes; 384 x 65536: 145.5 ->
-// 131.3 us).  Runtime plans transpose through shared memory
-// after the last pass.
+// (16384^2 bf16 along rows: 1047 -> 917 us for both passes; 384 x 65536: 145.5
+// -> 131.3 us).  Runtime plans transpose through shared memory after the last
+// pass.
 template <bool INV, class S, int MODE, class Plan, class In>
 __device__ __forceinline__ void fs_transform(const Plan& P, const FsPlace& pl, const FsArgs& a, const In& in, S* out,
                                              const Cx<float>* twl, int col, bool valid, Cx<float>* sm) {

@@ -305,8 +305,6 @@ bool factor_radices(int n, int maxe, std::vector<int>& radices, std::string& why
   return true;
 }
 
-int get_twiddle_table(int dev, int count, int den, bool f64, void** out) { return get_table(dev, count, den, f64, out); }
-
 int get_stage_table(int dev, const std::vector<int>& radices, bool f64, void** out) {
   return build_stage_table(dev, radices, f64, out);
 }
