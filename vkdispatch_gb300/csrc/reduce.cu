@@ -91,20 +91,31 @@ __device__ __forceinline__ T block_reduce(T v, T* sh) {
   return v;
 }
 
-// Stage 1: part p of row b covers elements [p*chunk, min(n, (p+1)*chunk)) and is
-// folded by W warps, about 64 elements per thread: a CTA of eight warps holds
-// 8 / W parts.  (One 512-thread CTA per part spent 16 instructions per element
-// on 4096-element parts, most of them on the block's fold: 1024 x 65536 floats
-// took 54.9 us, 46.3 us this way; 39.5 us is the copy rate.)  A thread takes
-// four neighbouring elements per step, in 16-byte loads where the part starts
-// on such a boundary and in single loads of the same elements otherwise, and
-// the fold's order depends on n alone, so results do too.
+// Stage 1: part p of row b covers elements [p*chunk, min(n, (p+1)*chunk)), in
+// blocks of 512 elements, 16 per lane of a warp.  Block k belongs to slot k % 8;
+// a lane folds the blocks of its slots, the slots are folded as a tree, and the
+// lanes last.  W warps (1 to 8) share a part's slots, and a CTA of eight warps
+// holds 8 / W parts.  That order depends on n alone, whatever W is, so results
+// do too, and W follows the amount of work: two warps per 4096 elements where
+// the parts fill the chip (one 512-thread CTA per part spent 16 instructions
+// per element, most of them on the fold: 1024 x 65536 floats took 54.9 us
+// against a copy rate of 39.5), eight where they do not (262144 complex
+// magnitudes on two warps a part took 11.4 us, their loads one after another).
+//
+// A lane's elements of a block are neighbours in fours where n is a multiple of
+// four, in 16-byte loads if the part starts on such a boundary; rows of another
+// n start at any element, so there each load of a warp is of neighbours (33 rows
+// of 1710185 complex elements: 94 us; 104 us in fours).
 constexpr int kWarps = 8;
 constexpr int kVec = 4;
+constexpr int kStep = 32 * kVec;   // elements of a warp per step
+constexpr int kBlock = 4 * kStep;  // elements of a block
+constexpr long long kFullWarps = 152 * 32;  // warps that fill the chip
 
-inline int part_warps(long long chunk) {
+inline int part_warps(long long chunk, long long parts) {
   int w = 1;
   while (w < kWarps && chunk > 64ll * 32 * w) w <<= 1;
+  while (w < kWarps && (long long)kBlock * w < chunk && parts * w < kFullWarps) w <<= 1;
   return w;
 }
 
@@ -120,56 +131,116 @@ __device__ __forceinline__ T warp_reduce(T v) {
   return v;
 }
 
+// A lane's fold of step k of a block; the first `left` elements count (all of
+// them if WHOLE).  pack: fours of neighbours; vec: q is aligned for 16-byte loads.
+template <class In, bool WHOLE>
+__device__ __forceinline__ void load_step(In (&x)[kVec], const In* __restrict__ q, int k, int left, bool pack, bool vec,
+                                          int lane) {
+  const int first = k * kStep + (pack ? lane * kVec : lane), de = pack ? 1 : 32;
+  if (vec) {
+    Pack<In> p4{};
+    if (WHOLE || first < left) p4 = *reinterpret_cast<const Pack<In>*>(q + first);
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) x[i] = p4.v[i];
+  } else {
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) x[i] = WHOLE || first + i * de < left ? q[first + i * de] : In{};
+  }
+}
+
+template <class In, class T, int OP, int MAP, bool WHOLE>
+__device__ __forceinline__ T fold_step(const In (&x)[kVec], int k, int left, bool pack, int lane) {
+  const int first = k * kStep + (pack ? lane * kVec : lane), de = pack ? 1 : 32;
+  T m[kVec];
+#pragma unroll
+  for (int i = 0; i < kVec; ++i)
+    m[i] = WHOLE || first + i * de < left ? apply_map<In, T, MAP>(x[i]) : identity<T, OP>();
+  return combine<T, OP>(combine<T, OP>(m[0], m[1]), combine<T, OP>(m[2], m[3]));
+}
+
+// A lane's fold of a block: the loads of all four steps first where the block is
+// whole; a part's last block goes step by step and stops with its elements.
+template <class In, class T, int OP, int MAP>
+__device__ __forceinline__ T fold_block(const In* __restrict__ q, long long len, bool pack, bool vec, int lane) {
+  if (len >= kBlock) {
+    In x[4][kVec];
+    if (vec) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) load_step<In, true>(x[k], q, k, kBlock, pack, true, lane);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) load_step<In, true>(x[k], q, k, kBlock, pack, false, lane);
+    }
+    T r[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) r[k] = fold_step<In, T, OP, MAP, true>(x[k], k, kBlock, pack, lane);
+    return combine<T, OP>(combine<T, OP>(r[0], r[1]), combine<T, OP>(r[2], r[3]));
+  }
+  const int left = (int)len;
+  T lower = identity<T, OP>(), pair = lower, r = lower;
+#pragma unroll 1
+  for (int k = 0; k * kStep < left; ++k) {
+    In x[kVec];
+    load_step<In, false>(x, q, k, left, pack, vec, lane);
+    r = fold_step<In, T, OP, MAP, false>(x, k, left, pack, lane);
+    if (k & 1) {
+      r = combine<T, OP>(pair, r);
+      if (k == 1) lower = r;
+      pair = identity<T, OP>();
+    } else {
+      pair = r;
+    }
+    if (k != 1) r = combine<T, OP>(lower, r);
+  }
+  return r;
+}
+
 template <class In, class T, int OP, int MAP>
 __global__ void __launch_bounds__(32 * kWarps) k_reduce_partial(const In* __restrict__ in, long long n, long long chunk,
                                                                 T* __restrict__ part, int nparts, int W) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int TH = 32 * W;  // threads of a part, a power of two
-  __shared__ T sh[kWarps];
-  const int g = threadIdx.x / TH, t = threadIdx.x & (TH - 1);
+  __shared__ T sh[kWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int w = warp & (W - 1);  // warp of its part; W is a power of two
   const long long b = blockIdx.y;
-  const int p = blockIdx.x * (kWarps / W) + g;
-  T a[kVec];
-#pragma unroll
-  for (int i = 0; i < kVec; ++i) a[i] = identity<T, OP>();
-  const In* row = in + b * n;
+  const int p = blockIdx.x * (kWarps / W) + warp / W;
   const long long lo = (long long)p * chunk;
-  long long hi = lo + chunk;
-  if (hi > n) hi = n;
-  if (p < nparts) {
-    const In* q = row + lo;
-    const long long full = hi > lo ? (hi - lo) / (kVec * TH) : 0;  // whole steps of the part's threads
-    if (reinterpret_cast<unsigned long long>(q) % alignof(Pack<In>) == 0) {
-      const Pack<In>* v = reinterpret_cast<const Pack<In>*>(q) + t;
-#pragma unroll 4
-      for (long long s = 0; s < full; ++s) {
-        const Pack<In> x = v[s * TH];
-#pragma unroll
-        for (int i = 0; i < kVec; ++i) a[i] = combine<T, OP>(a[i], apply_map<In, T, MAP>(x.v[i]));
-      }
-    } else {
-#pragma unroll 4
-      for (long long s = 0; s < full; ++s) {
-        In x[kVec];
-#pragma unroll
-        for (int i = 0; i < kVec; ++i) x[i] = q[(s * TH + t) * kVec + i];
-#pragma unroll
-        for (int i = 0; i < kVec; ++i) a[i] = combine<T, OP>(a[i], apply_map<In, T, MAP>(x[i]));
+  const long long len = (lo + chunk < n ? lo + chunk : n) - lo;
+  T acc = identity<T, OP>();
+  if (p < nparts && len > 0) {
+    const In* q = in + b * n + lo;
+    const bool pack = n % kVec == 0;
+    const bool vec = pack && reinterpret_cast<unsigned long long>(q) % alignof(Pack<In>) == 0;
+    const int slots = kWarps / W;
+    T h1 = acc, h2 = acc, h4 = acc;  // finished lower halves of the slots' tree
+    for (int j = 0; j < slots; ++j) {
+      T v = identity<T, OP>();
+      for (long long e = (long long)(w * slots + j) * kBlock; e < len; e += kWarps * kBlock)
+        v = combine<T, OP>(v, fold_block<In, T, OP, MAP>(q + e, len - e, pack, vec, lane));
+      if (slots == 1) acc = v;
+      else if (!(j & 1)) h1 = v;
+      else {
+        v = combine<T, OP>(h1, v);
+        if (slots == 2) acc = v;
+        else if (!(j & 2)) h2 = v;
+        else {
+          v = combine<T, OP>(h2, v);
+          if (slots == 4) acc = v;
+          else if (!(j & 4)) h4 = v;
+          else acc = combine<T, OP>(h4, v);
+        }
       }
     }
-    for (long long e = lo + full * kVec * TH + t; e < hi; e += TH)
-      a[0] = combine<T, OP>(a[0], apply_map<In, T, MAP>(row[e]));
   }
-  T acc = combine<T, OP>(combine<T, OP>(a[0], a[1]), combine<T, OP>(a[2], a[3]));
-  acc = warp_reduce<T, OP>(acc);
-  if (W > 1) {
-    const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) sh[w] = acc;
+  for (int d = 1; d < W; d <<= 1) {  // the upper levels of the slots' tree, across the part's warps
+    sh[warp][lane] = acc;
     __syncthreads();
-    if (t == 0)
-      for (int i = 1; i < W; ++i) acc = combine<T, OP>(acc, sh[w + i]);
+    if ((w & (2 * d - 1)) == 0) acc = combine<T, OP>(acc, sh[warp + d][lane]);
+    __syncthreads();
   }
-  if (t == 0 && p < nparts) part[b * nparts + p] = acc;
+  if (w != 0) return;
+  acc = warp_reduce<T, OP>(acc);
+  if (lane == 0 && p < nparts) part[b * nparts + p] = acc;
 }
 
 // Stage 2 folds the partials of a row in a fixed order: one warp per row for
@@ -200,7 +271,7 @@ template <class In, class T, int OP, int MAP>
 cudaError_t run(const void* in, long long n, long long batch, void* out, void* partials, int nparts, cudaStream_t s) {
   // parts start on 16-byte steps of the row
   const long long chunk = ((n + nparts - 1) / nparts + 3) & ~3ll;
-  const int W = part_warps(chunk), G = kWarps / W;
+  const int W = part_warps(chunk, nparts * batch), G = kWarps / W;
   const Launch l1{dim3((unsigned)((nparts + G - 1) / G), (unsigned)batch), dim3(32 * kWarps), 0, s};
   const In* src = reinterpret_cast<const In*>(in);
   T* part = reinterpret_cast<T*>(partials);
