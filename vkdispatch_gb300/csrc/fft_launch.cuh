@@ -146,6 +146,9 @@ cudaError_t launch_with_plan(const FftArgs& a, const Launch& l, int op, bool str
 
 template <class S, class Re>
 cudaError_t launch_fft(const FftArgs& a, const Launch& l, int op, bool strided, int kop, int variant) {
+  // radix_dispatch ends at 16: a pass of a larger radix would do nothing
+  for (int q = 0; q < a.pp.npass; ++q)
+    if (a.pp.radix[q] > 16) return cudaErrorInvalidValue;
   if (variant != 0 && op != OP_C2C_FWD && op != OP_C2C_INV && op != OP_CONV) return cudaErrorInvalidValue;
   switch (op) {
     case OP_C2C_FWD:

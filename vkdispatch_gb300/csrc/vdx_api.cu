@@ -344,6 +344,7 @@ struct Tune {
   int fixed = -1;     // compile-time kernels where available: -1 = yes, 0 = no
   int fourstep = -1;  // long C2C axes: -1 = from 8192 points (VDX_FOURSTEP_MIN), 0 = only above one CTA, 1 = always
   int maxe = 0;       // points per thread: 0 = the plan's default, or 16 / 8 / 32 (compile-time plans where they exist)
+  int points = 8 | 16 | 32;  // points per thread that the default and VDX_POINTS_PER_THREAD may choose
 };
 }  // namespace vdx
 
@@ -896,8 +897,10 @@ int plan_bluestein(const vdx_fft_desc& d, long long inner, long long outer, int 
   dc.kernel_broadcast = 1;
   int rc = VDX_OK;
   if (!split) {
+    // the plan's radix list runs on the storage type's kernels: other storage
+    // than complex64 has none of 8 or 32 points per thread
     Tune t;
-    if (st != ST_C64) t.maxe = 16;  // the two-pass radix-32 plans exist for complex64 storage
+    if (st != ST_C64) t.points = 16;
     rc = create_plan(&dc, t, &p->bs_conv);
   } else {
     dc.kind = VDX_KIND_C2C;
@@ -1038,13 +1041,13 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
   // 82.1, 32768 x 512 rows 89.9 -> 72.5); rows of C2C are indifferent (85.9 ->
   // 85.0, 84.5 -> 86.5) and 1024-point convolutions along rows lose (96.2 ->
   // 118.6)
-  if (tune.maxe == 0 && !real && canpts && has_fixedpts_c64(n, 32, is_conv, inner > 1) &&
+  if (tune.maxe == 0 && (tune.points & 32) && !real && canpts && has_fixedpts_c64(n, 32, is_conv, inner > 1) &&
       (inner > 1 || (is_conv && n == 512)))
     pmaxe = 32;
   if (const char* e = std::getenv("VDX_POINTS_PER_THREAD")) {
     const int v = std::atoi(e);
     if (v == 16) pmaxe = 16;
-    if ((v == 8 || v == 32) && canpts && has_fixedpts_c64(n, v, is_conv, inner > 1)) pmaxe = v;
+    if ((v == 8 || v == 32) && (tune.points & v) && canpts && has_fixedpts_c64(n, v, is_conv, inner > 1)) pmaxe = v;
   }
   if (pmaxe != 16 && !(canpts && has_fixedpts_c64(n, pmaxe, is_conv, inner > 1))) {
     delete p;
