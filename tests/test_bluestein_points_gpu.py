@@ -8,7 +8,7 @@ import pytest
 import vkdispatch_gb300 as vd
 from vkdispatch_gb300.fft import plan as P
 
-from helpers import crandn, rel_l2
+from helpers import crandn, rel_l2, tol_fp32
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +38,9 @@ def _check(n, storage, tol):
 @pytest.mark.parametrize("n", [131, 262, 509])
 def test_half_storage(choice, n, storage, tol):
     _check(n, storage, tol)
+
+
+@pytest.mark.parametrize("n", [131, 211, 262, 509])
+def test_c64(choice, n):
+    # forward and inverse convolutions of the chirp at up to 4n points
+    _check(n, vd.complex64, 3 * tol_fp32(4 * n))

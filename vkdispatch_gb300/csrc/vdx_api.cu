@@ -897,10 +897,10 @@ int plan_bluestein(const vdx_fft_desc& d, long long inner, long long outer, int 
   dc.kernel_broadcast = 1;
   int rc = VDX_OK;
   if (!split) {
-    // the plan's radix list runs on the storage type's kernels: other storage
-    // than complex64 has none of 8 or 32 points per thread
+    // the plan's radix list runs on the storage type's Bluestein kernels: none
+    // has 8 points per thread, and only complex64 has 32
     Tune t;
-    if (st != ST_C64) t.points = 16;
+    t.points = st == ST_C64 ? 16 | 32 : 16;
     rc = create_plan(&dc, t, &p->bs_conv);
   } else {
     dc.kind = VDX_KIND_C2C;
