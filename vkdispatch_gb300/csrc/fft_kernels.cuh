@@ -667,6 +667,27 @@ __device__ __forceinline__ void pass_tail(PassAt a, Slots<Re, PADDED> x, const C
   each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { out.template store<R>(&v[b * R], j, a.nb); });
 }
 
+// pass_mid or, for the plan's last pass, pass_tail in one body
+template <int R, int MAXE, bool INV, class Re, bool PADDED, class Out>
+__device__ __forceinline__ void pass_rest(PassAt a, Slots<Re, PADDED> x, const Cx<Re>* tw, const Out& out, bool last,
+                                          bool smout) {
+  Values<MAXE, Re> w;
+  Cx<Re>* v = w.v;
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { x.template load<R>(&v[b * R], j, a.nb); });
+  each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { twiddled_dft<R, INV>(&v[b * R], a.k(j), a.ns, tw); });
+  if (last) {
+    if (smout) xsync(a.warp);
+    each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) { out.template store<R>(&v[b * R], j, a.nb); });
+  } else {
+    xsync(a.warp);
+    each_butterfly<R, MAXE>(a.nb, a.T, a.t, [&](auto b, int j) {
+      const int k = a.k(j);
+      x.template store<R>(&v[b * R], (j - k) * R + k, a.ns);
+    });
+    xsync(a.warp);
+  }
+}
+
 // source -> sink (a plan of one pass: one thread holds a whole transform)
 template <int R, int MAXE, bool INV, class Re, class In, class Out>
 __device__ __forceinline__ void pass_only(PassAt a, const In& in, const Out& out) {
@@ -751,6 +772,32 @@ __device__ __forceinline__ void runtime_transform(const PassPlan& pp, int t, con
   });
 }
 
+// The same with one body per radix for the middle and the last pass.
+template <int MAXE, bool INV, class Re, bool PADDED, class In, class Out>
+__device__ __forceinline__ void merged_transform(const PassPlan& pp, int t, const Slots<Re, PADDED>& x,
+                                                 const Cx<Re>* tw, const In& in, const Out& out, bool smin, bool smout,
+                                                 bool warp) {
+  const int P = pp.npass, R0 = pp.radix[0];
+  if (P > 1) {
+    radix_dispatch(R0, [&](auto rc) {
+      pass_head<decltype(rc)::value, MAXE, INV>(pass_at<false>(pp, 0, 1, t, warp), x, in, smin);
+    });
+  } else {
+    radix_dispatch(R0, [&](auto rc) {
+      pass_only<decltype(rc)::value, MAXE, INV, Re>(pass_at<false>(pp, 0, 1, t, warp), in, out);
+    });
+    return;
+  }
+  int ns = R0;
+  for (int q = 1; q < P; ++q) {
+    const int R = pp.radix[q];
+    radix_dispatch(R, [&](auto rc) {
+      pass_rest<decltype(rc)::value, MAXE, INV>(pass_at<false>(pp, q, ns, t, warp), x, tw, out, q + 1 == P, smout);
+    });
+    ns *= R;
+  }
+}
+
 // Forward transform, spectrum operation, inverse transform with the passes
 // reversed.
 template <int MAXE, class Re, bool PADDED, class In, class Op, class Out>
@@ -811,10 +858,14 @@ struct RRev<RList<>, RList<Os...>> {
   using type = RList<Os...>;
 };
 
-template <int MAXE_, bool PAD_ = true>
+// MERGED: the middle and the last pass of a transform share one body per radix,
+// so a list of equal radices runs the same instructions again instead of
+// fetching others; the body needs more registers.
+template <int MAXE_, bool PAD_ = true, bool MERGED_ = false>
 struct DynPlan {
   static constexpr int MAXE = MAXE_;
   static constexpr bool PAD = PAD_;
+  static constexpr bool kMerged = MERGED_;
   __device__ __forceinline__ void assume_t(int) const {}
   const PassPlan& pp;
   __device__ __forceinline__ explicit DynPlan(const PassPlan& p) : pp(p) {}
@@ -842,8 +893,9 @@ struct DynPlan {
   template <bool INV, bool SMIN, bool SMOUT, class PL, class Re, class In, class Out>
   __device__ __forceinline__ void transform(const PL& pl, Cx<Re>* sm, const Cx<Re>* tw, const In& in,
                                             const Out& out) const {
-    runtime_transform<MAXE, INV>(pp, pl.t, slots<Re>(pl, sm), tw, in, out, SMIN, SMOUT,
-                                 WarpLocal<PL>::value && warp_sized(pp.T));
+    const bool warp = WarpLocal<PL>::value && warp_sized(pp.T);
+    if constexpr (kMerged) merged_transform<MAXE, INV>(pp, pl.t, slots<Re>(pl, sm), tw, in, out, SMIN, SMOUT, warp);
+    else runtime_transform<MAXE, INV>(pp, pl.t, slots<Re>(pl, sm), tw, in, out, SMIN, SMOUT, warp);
   }
   template <class PL, class Re, class In, class Op, class Out>
   __device__ __forceinline__ void convolve(const PL& pl, Cx<Re>* sm, const Cx<Re>* tw, const Cx<Re>* twr,
@@ -882,6 +934,7 @@ template <int N_, int T_, class L, int MAXE_ = 16>
 struct FixPlan {
   static constexpr int MAXE = MAXE_;
   static constexpr bool PAD = true;
+  static constexpr bool kMerged = false;
   static constexpr int kFirst = RFirst<L>::value, kLast = RLast<L>::value;
   // the thread's index inside its transform is below T (lets the compiler
   // drop the j < n/R guards of exact plans)

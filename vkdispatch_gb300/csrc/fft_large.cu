@@ -24,11 +24,12 @@ namespace vdx {
 
 int fourstep_pitch(const PassPlan& pp) { return fs_pitch(pp.M, pp.T); }
 
-cudaError_t launch_fourstep_pass(const FsArgs& a, const Launch& l, int store, bool inv, int mode) {
+cudaError_t launch_fourstep_pass(const FsArgs& a, const Launch& l, int store, bool inv, int mode, bool few) {
+  few = few && !fourstep_fixed(a.pp);
   switch (store) {
-    case ST_C64: return launch_fs_c64(a, l, inv, mode);
-    case ST_C32: return launch_fs_c32(a, l, inv, mode);
-    case ST_BF16: return launch_fs_bf16(a, l, inv, mode);
+    case ST_C64: return few ? launch_fs_few_c64(a, l, inv, mode) : launch_fs_c64(a, l, inv, mode);
+    case ST_C32: return few ? launch_fs_few_c32(a, l, inv, mode) : launch_fs_c32(a, l, inv, mode);
+    case ST_BF16: return few ? launch_fs_few_bf16(a, l, inv, mode) : launch_fs_bf16(a, l, inv, mode);
     default: return cudaErrorInvalidValue;
   }
 }

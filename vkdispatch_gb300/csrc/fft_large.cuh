@@ -123,8 +123,10 @@ __device__ __forceinline__ void fs_transpose(const Plan& P, const FsPlace& pl, c
   });
 }
 
+// Registers: 64 a thread (two CTAs of 512), or 128 on a merged plan, which the
+// launches take whose CTAs all run at once (see fourstep_few).
 template <class Plan, bool INV, class S, int MODE>
-__global__ void __launch_bounds__(512, 2) k_fs(FsArgs a) {
+__global__ void __launch_bounds__(512, Plan::kMerged ? 1 : 2) k_fs(FsArgs a) {
   using Re = float;
   const Plan P(a.pp);
   const int M = a.pp.M;
@@ -186,9 +188,18 @@ cudaError_t launch_any(const FsArgs& a, const Launch& l, bool inv, int mode) {
   return launch_mode<DynPlan<16, false>, S>(a, l, inv, mode);
 }
 
-// the instantiations of one storage type (fft_large_c64.cu, _c32.cu, _bf16.cu)
+template <class S>
+cudaError_t launch_few(const FsArgs& a, const Launch& l, bool inv, int mode) {
+  return launch_mode<DynPlan<16, false, true>, S>(a, l, inv, mode);
+}
+
+// the instantiations of one storage type (fft_large_c64.cu, _c32.cu, _bf16.cu,
+// and fft_large_few_*.cu)
 cudaError_t launch_fs_c64(const FsArgs& a, const Launch& l, bool inv, int mode);
 cudaError_t launch_fs_c32(const FsArgs& a, const Launch& l, bool inv, int mode);
 cudaError_t launch_fs_bf16(const FsArgs& a, const Launch& l, bool inv, int mode);
+cudaError_t launch_fs_few_c64(const FsArgs& a, const Launch& l, bool inv, int mode);
+cudaError_t launch_fs_few_c32(const FsArgs& a, const Launch& l, bool inv, int mode);
+cudaError_t launch_fs_few_bf16(const FsArgs& a, const Launch& l, bool inv, int mode);
 
 }  // namespace vdx

@@ -372,6 +372,7 @@ struct vdx_plan {
   FsArgs fsA{}, fsB{};  // pass plans, twiddles and scale; geometry is set per chunk
   dim3 blockA, blockB;
   size_t smemA = 0, smemB = 0;
+  int sms = 1;  // of the plan's device
   void* ws = nullptr;
   size_t ws_bytes = 0;
   // both passes in one persistent launch with an L2-resident ring (fft_fused4.cu)
@@ -622,6 +623,7 @@ int plan_fourstep(vdx_plan* p, long long inner, long long outer, int smem_optin)
     p->chunk_outer = R;
     p->ws_bytes = size_t(R) * size_t(col_bytes);
   }
+  cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->dev);
   p->fourstep = true;
   p->N1 = N1;
   p->N0 = N0;
@@ -779,7 +781,7 @@ cudaError_t exec_fourstep(const vdx_plan* p, const void* in, void* out, cudaStre
         A.nbatch = Oc * N0;
         la.grid = dim3((unsigned)(Oc * N0 * A.col_tiles));
         e = p->tensor_core ? launch_fourstep_pass_tc(A, la, p->store, inv, 1, p->tc_bmat, p->d_status)
-                           : launch_fourstep_pass(A, la, p->store, inv, 1);
+                           : launch_fourstep_pass(A, la, p->store, inv, 1, fourstep_few(la, p->sms));
         if (e != cudaSuccess) return e;
         FsArgs B = p->fsB;
         B.in = p->ws;
@@ -797,7 +799,7 @@ cudaError_t exec_fourstep(const vdx_plan* p, const void* in, void* out, cudaStre
         B.nbatch = Oc * N1;
         lb.grid = dim3((unsigned)(Oc * N1 * B.col_tiles));
         e = p->tensor_core ? launch_fourstep_pass_tc(B, lb, p->store, inv, 0, p->tc_bmat, p->d_status)
-                           : launch_fourstep_pass(B, lb, p->store, inv, 0);
+                           : launch_fourstep_pass(B, lb, p->store, inv, 0, fourstep_few(lb, p->sms));
         if (e != cudaSuccess) return e;
       }
     }
@@ -823,7 +825,7 @@ cudaError_t exec_fourstep(const vdx_plan* p, const void* in, void* out, cudaStre
     A.nbatch = Rr;
     la.grid = dim3((unsigned)(Rr * A.col_tiles));
     e = p->tensor_core ? launch_fourstep_pass_tc(A, la, p->store, inv, 2, p->tc_bmat, p->d_status)
-                       : launch_fourstep_pass(A, la, p->store, inv, 2);
+                       : launch_fourstep_pass(A, la, p->store, inv, 2, fourstep_few(la, p->sms));
     if (e != cudaSuccess) return e;
     FsArgs B = p->fsB;
     B.in = p->ws;
@@ -841,7 +843,7 @@ cudaError_t exec_fourstep(const vdx_plan* p, const void* in, void* out, cudaStre
     B.nbatch = Rr;
     lb.grid = dim3((unsigned)(Rr * B.col_tiles));
     e = p->tensor_core ? launch_fourstep_pass_tc(B, lb, p->store, inv, 0, p->tc_bmat, p->d_status)
-                       : launch_fourstep_pass(B, lb, p->store, inv, 0);
+                       : launch_fourstep_pass(B, lb, p->store, inv, 0, fourstep_few(lb, p->sms));
     if (e != cudaSuccess) return e;
   }
   return e;

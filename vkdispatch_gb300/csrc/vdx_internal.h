@@ -95,7 +95,18 @@ inline bool fourstep_fixed(const PassPlan& pp) {
   return (pp.n == 128 && pp.T == 8) || (pp.n == 256 && pp.T == 16) || (pp.n == 64 && pp.T == 4);
 }
 int fourstep_pitch(const PassPlan& pp);
-cudaError_t launch_fourstep_pass(const FsArgs& a, const Launch& l, int store, bool inv, int mode);
+// Whether every CTA of a launch runs at once at 128 registers a thread (512
+// threads an SM).  Such a launch waits for instructions and loads, not for
+// issue slots: its runtime plans take a kernel of twice the registers, without
+// spills, whose middle and last passes share their code (one 8575-point row
+// 20.1 us for both passes with 64 registers, 17.1 with 128; 1 x 16807 x 4 18.3
+// and 14.8, 1 x 28561 x 4 17.1 and 13.0).  Launches of more CTAs lose their
+// second CTA per SM by it (1 x 240240 x 4: 22.4 and 27.0).
+inline bool fourstep_few(const Launch& l, int sms) {
+  const int per_sm = 512 / (((int)l.block.x + 31) / 32 * 32);
+  return (long long)l.grid.x <= (long long)per_sm * sms;
+}
+cudaError_t launch_fourstep_pass(const FsArgs& a, const Launch& l, int store, bool inv, int mode, bool few);
 // The same pass with the 128-point short transforms on the tensor cores
 // (fft_tc.cu); a.pp.n must be 128 and a.pp.M 16 or 32.  bmat = the DFT
 // operand image from tc_dft_operands; *status is set to 1 if an MMA
