@@ -1153,12 +1153,13 @@ __global__ void __launch_bounds__(256, Plan::MAXE <= 8 ? 3 : 2) k_conv_pf(FftArg
     });
   }
   Plan::template each<RR>(pl.t, [&](auto b, int j) {
-    const S* q = ker + j * pl.ps;
+    // no stepping pointer: 32 addresses in a chain keep the loads from going out
+    // together (64 x 1024 x 512 along axis 1: 260.8 -> 181.7 us)
 #pragma unroll
-    for (int r = 0; r < RR; ++r, q += step) {
+    for (int r = 0; r < RR; ++r) {
       Cx<Re> k;
       if constexpr (PF) k = kr[b * RR + r];
-      else k = kvalid ? ld_once<S, Re>(q) : mk<Re>(Re(0), Re(0));
+      else k = kvalid ? ld_once<S, Re>(ker + (j + r * nb) * pl.ps) : mk<Re>(Re(0), Re(0));
       v[b * RR + r] = KOP == 0 ? cmulc(v[b * RR + r], k) : cmul(v[b * RR + r], k);
     }
   });

@@ -46,10 +46,11 @@ cudaError_t launch_conv_layout(const FftArgs& a, const Launch& l, int variant) {
   if constexpr (C64 && IsFixPlan<Plan>::value) {
     // 32-point plans have no registers for early loads, so for them k_conv_pf only
     // differs in reading the spectrum evict-first: right for one that each image
-    // has of its own (64 x 512 x 512 images: 83.9 -> 81.9 us), wrong for one that
-    // all share and L2 should keep (40 x 1024 x 256: 75.8 -> 81.9), and slower at
-    // 1024 points either way (147 x 1024 x 64: 108.6 -> 112.6).
-    const bool early = Plan::MAXE <= 16 || (a.ker_bs != 0 && a.pp.n < 1024);
+    // has of its own (64 x 512 x 512 images: 83.9 -> 81.9 us; 16 x 1024 x 513 along
+    // axis 1: 74.1 -> 48.8), wrong for one that all share and L2 should keep
+    // (40 x 1024 x 256: 75.8 -> 81.9), and at 1024 points wrong where the forward
+    // spectrum is written too (64 x 1024 x 33: 24.2 -> 45.5).
+    const bool early = Plan::MAXE <= 16 || (a.ker_bs != 0 && (variant == 0 || a.pp.n < 1024));
     if (l.block.x <= 256 && early && conv_prefetch()) {
       if (variant == 0) return enqueue_pdl(k_conv_pf<Plan, STRIDED, S, Re, KOP>, l, a);
       if constexpr (KOP == 0) {
