@@ -1,0 +1,47 @@
+"""Plans of lengths whose radices are all even: the pass whose scatter conflicts
+least runs first, in every kernel that runs the list."""
+
+import numpy as np
+import pytest
+
+import vkdispatch_gb300 as vd
+from vkdispatch_gb300 import _lib as L
+from vkdispatch_gb300.fft import plan as P
+
+from helpers import crandn, rel_l2, tol_fp32
+
+pytestmark = pytest.mark.gpu
+
+
+def _plan(shape, axis=1):
+    return P.get_plan(shape, axis, L.VDX_KIND_C2C, False, False, L.VDX_C64, L.VDX_C64).describe()
+
+
+@pytest.mark.parametrize("n,first", [(2304, 12), (2688, 14), (2240, 14), (144, 12), (80, 10)])
+def test_first_radix(n, first):
+    radices = [int(r) for r in _plan((64, n))["radices"].split("x")]
+    assert int(np.prod(radices)) == n
+    if all(r % 2 == 0 for r in radices):
+        assert radices[0] == first
+
+
+@pytest.mark.parametrize("n", [144, 192, 1000, 2240, 2304, 2688])
+def test_transforms(n):
+    rng = np.random.default_rng(n)
+    for shape, axis in (((5, n), 1), ((2, n, 11), 1)):
+        x, k = crandn(rng, shape), crandn(rng, shape)
+        b = vd.asbuffer(x)
+        vd.fft.fft(b, axis=axis)
+        want = np.fft.fft(x.astype(np.complex128), axis=axis)
+        assert rel_l2(b.read(0), want) <= tol_fp32(n)
+        vd.fft.ifft(b, axis=axis)
+        assert rel_l2(b.read(0), x) <= 2 * tol_fp32(n)
+        c = vd.asbuffer(x)
+        vd.fft.convolve(c, vd.asbuffer(k), axis=axis)
+        assert rel_l2(c.read(0), np.fft.ifft(want * np.conj(k), axis=axis)) <= 2 * tol_fp32(n)
+    r = rng.standard_normal((5, 2 * n)).astype(np.float32)
+    rb = vd.asrfftbuffer(r)
+    vd.fft.rfft(rb)
+    assert rel_l2(rb.read_fourier(0), np.fft.rfft(r.astype(np.float64), axis=-1)) <= tol_fp32(2 * n)
+    vd.fft.irfft(rb)
+    assert rel_l2(rb.read_real(0), r) <= 2 * tol_fp32(2 * n)

@@ -299,8 +299,17 @@ bool factor_radices(int n, int maxe, std::vector<int>& radices, std::string& why
       best = s.best;
     }
     radices = best;
-    auto odd = std::find_if(radices.begin(), radices.end(), [](int r) { return r % 2 == 1; });
-    if (odd != radices.end()) std::rotate(radices.begin(), odd, odd + 1);
+    // first the radix R with the fewest factors of two: the first scatter of a
+    // row steps by R slots of two banks, 16-way conflicts for 16, 4-way for 12,
+    // 2-way for 10 and 14, none for odd ones (3640 rows of 2304 points 54.4 us
+    // as 16 x 12 x 12, 34.6 as 12 x 16 x 12; 3120 of 2688 58.8 as 16 x 14 x 12, 35.3
+    // as 14 x 16 x 12).  Lists of 16s and one other radix keep the 16s first:
+    // their rows are padded (PassPlan::pad)
+    auto twos = [](int r) { return r & -r; };
+    if (std::count(radices.begin(), radices.end(), 16) + 1 < (long)radices.size() || radices.back() % 2 == 1) {
+      auto first = std::min_element(radices.begin(), radices.end(), [&](int x, int y) { return twos(x) < twos(y); });
+      std::rotate(radices.begin(), first, first + 1);
+    }
   }
   return true;
 }
