@@ -1,5 +1,6 @@
-"""Plans of lengths whose radices are all even: the pass whose scatter conflicts
-least runs first, in every kernel that runs the list."""
+"""Choices of the planner for runtime lengths, and the kernels on them: in lists
+of even radices the pass whose scatter conflicts least runs first; rows of 33 to
+48 threads share a CTA where they are short."""
 
 import numpy as np
 import pytest
@@ -45,3 +46,22 @@ def test_transforms(n):
     assert rel_l2(rb.read_fourier(0), np.fft.rfft(r.astype(np.float64), axis=-1)) <= tol_fp32(2 * n)
     vd.fft.irfft(rb)
     assert rel_l2(rb.read_real(0), r) <= 2 * tol_fp32(2 * n)
+
+
+@pytest.mark.parametrize("n,rows_per_cta", [(297, 3), (363, 3), (405, 2), (504, 1), (546, 1)])
+def test_rows_per_cta(n, rows_per_cta):
+    d = _plan((200, n))
+    if 32 < d["threads_per_transform"] <= 48:
+        assert d["transforms_per_cta"] == rows_per_cta
+    rng = np.random.default_rng(n)
+    for rows in (1, 2, 7):
+        x = crandn(rng, (rows, n))
+        b = vd.asbuffer(x)
+        vd.fft.fft(b)
+        assert rel_l2(b.read(0), np.fft.fft(x.astype(np.complex128))) <= tol_fp32(n)
+        vd.fft.ifft(b)
+        assert rel_l2(b.read(0), x) <= 2 * tol_fp32(n)
+    r = rng.standard_normal((7, 2 * n)).astype(np.float32)
+    rb = vd.asrfftbuffer(r)
+    vd.fft.rfft(rb)
+    assert rel_l2(rb.read_fourier(0), np.fft.rfft(r.astype(np.float64), axis=-1)) <= tol_fp32(2 * n)

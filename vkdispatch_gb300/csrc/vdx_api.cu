@@ -1152,9 +1152,17 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
     // the CTA's barriers (100000 x 360: 150 us with 128 threads, 138 with 64;
     // transforms inside one warp are indifferent)
     int cta_threads = 64;
-    if (const char* e = std::getenv("VDX_CTA_THREADS")) cta_threads = std::max(32, std::min(1024, std::atoi(e)));
+    const char* env = std::getenv("VDX_CTA_THREADS");
+    const bool asked = env || tune.width > 0;
+    if (env) cta_threads = std::max(32, std::min(1024, std::atoi(env)));
     if (tune.width > 0) cta_threads = std::max(32, std::min(1024, tune.width));
     M = std::max(1, cta_threads / T);
+    // one row of 33 to 48 threads leaves up to half of its second warp idle: two
+    // or three rows where a thread holds few points (3530 x 297: 10.0 us with one
+    // row of 33 threads, 7.8 with three; 59 such shapes 1.24 times as fast, none
+    // slower).  Longer rows are as fast or faster alone (2080 x 504, 42 threads of
+    // 12 points: 0.92 with three rows)
+    if (!asked && T > 32 && T <= 48 && n <= (T <= 36 ? 11 : 10) * T) M = 128 / T;
     M = (int)std::min<long long>(M, ntrans);
     M = std::max(1, std::min(M, (pmaxe == 32 ? 256 : 1024) / T));  // 32-point plans: CTAs of <= 256 threads
     while (M > 1 && need_smem && size_t(npad) * M * cbytes > size_t(smem_optin) / 2) M /= 2;
