@@ -247,8 +247,7 @@ __device__ __forceinline__ int mod_inv(int j, int d, unsigned m) {
   return j - int(__umulhi(unsigned(j), m)) * d;
 }
 
-// RT: ns is a runtime value with nsm = inv_magic(ns); otherwise ns is a
-// compile-time constant and j % ns folds.
+// ns is a compile-time constant, so j % ns folds.
 // tw is stage-ordered: entry k + r ns of a pass holds W_{ns R}^{k r}, so the
 // lanes of a warp (consecutive j, hence consecutive k) read neighbouring
 // entries.  A natural table W_n^i is read at k r n/(ns R) instead, a stride
@@ -257,16 +256,15 @@ __device__ __forceinline__ int mod_inv(int j, int d, unsigned m) {
 // table, 78.8 us from a stage-ordered one, which is the copy bandwidth; the
 // 2048-point convolutions of 4096 x 1009 Bluestein rows: 123.9 -> 96.8 us
 // with their chirp launches).
-template <int R, int MAXE, bool INV, class Re, bool RT = false>
-__device__ __forceinline__ void butterflies(Cx<Re>* v, int nb, int T, int t, int ns, const Cx<Re>* tw,
-                                            unsigned nsm = 0) {
+template <int R, int MAXE, bool INV, class Re>
+__device__ __forceinline__ void butterflies(Cx<Re>* v, int nb, int T, int t, int ns, const Cx<Re>* tw) {
   constexpr int B = MAXE / R;
 #pragma unroll
   for (int b = 0; b < B; ++b) {
     const int j = t + b * T;
     if (j < nb) {
       if (ns > 1) {
-        const int k = RT ? mod_inv(j, ns, nsm) : j % ns;
+        const int k = j % ns;
 #pragma unroll
         for (int r = 1; r < R; ++r) {
           const Cx<Re> w = ldg(&tw[k + r * ns]);
@@ -275,56 +273,6 @@ __device__ __forceinline__ void butterflies(Cx<Re>* v, int nb, int T, int t, int
       }
       Dft<R, INV, Re>::run(&v[b * R]);
     }
-  }
-}
-
-template <int R, int MAXE, class Re, bool RT = false, class G>
-__device__ __forceinline__ void scatter(const Cx<Re>* v, int nb, int T, int t, int ns, G&& g, unsigned nsm = 0) {
-  constexpr int B = MAXE / R;
-#pragma unroll
-  for (int b = 0; b < B; ++b) {
-    const int j = t + b * T;
-    if (j < nb) {
-      const int k = RT ? (ns > 1 ? mod_inv(j, ns, nsm) : 0) : j % ns;
-      const int base = (j - k) * R + k;
-#pragma unroll
-      for (int r = 0; r < R; ++r) g(base + r * ns, v[b * R + r]);
-    }
-  }
-}
-
-// Runs every pass on v, which must already hold the inputs of the first
-// executed pass.  reversed = run radices last-to-first.  Returns with v
-// holding natural-order outputs laid out for the last executed radix.
-template <int MAXE, bool INV, class PL, class Re>
-__device__ __forceinline__ void run_passes(Cx<Re>* v, const PassPlan& pp, bool reversed, const PL& pl,
-                                           Cx<Re>* sm, const Cx<Re>* tw, bool warp = false) {
-  const int n = pp.n, P = pp.npass, T = pp.T, t = pl.t;
-  int ns = 1;
-  for (int q = 0; q < P; ++q) {
-    const int p = reversed ? P - 1 - q : q;
-    const int R = pp.radix[p];
-    const bool more = q + 1 < P;
-    const unsigned nsm = reversed ? pp.nsmr[q] : pp.nsm[q];
-    // one radix dispatch per pass covers the butterflies and the scatter
-    radix_dispatch(R, [&](auto rc) {
-      constexpr int RR = decltype(rc)::value;
-      butterflies<RR, MAXE, INV, Re, true>(v, n / RR, T, t, ns, tw, nsm);
-      if (more) {
-        xsync(warp);
-        scatter<RR, MAXE, Re, true>(
-            v, n / RR, T, t, ns, [&](int pos, Cx<Re> val) { sm[pl.sidx(pp, pos)] = val; }, nsm);
-      }
-    });
-    if (more) {
-      xsync(warp);
-      const int R2 = pp.radix[reversed ? P - 2 - q : q + 1];
-      radix_dispatch(R2, [&](auto rc) {
-        constexpr int RR = decltype(rc)::value;
-        gather<RR, MAXE, Re>(v, n / RR, T, t, [&](int pos) { return sm[pl.sidx(pp, pos)]; });
-      });
-    }
-    ns *= R;
   }
 }
 
@@ -824,6 +772,27 @@ __device__ __forceinline__ void runtime_convolve(const PassPlan& pp, int t, cons
   });
 }
 
+// The inverse transform alone with the passes reversed, from a source in shared
+// memory that an earlier transform's exchange may still be read from.
+template <int MAXE, class Re, bool PADDED, class In, class Out>
+__device__ __forceinline__ void runtime_inverse_reversed(const PassPlan& pp, int t, const Slots<Re, PADDED>& x,
+                                                         const Cx<Re>* twr, const In& in, const Out& out, bool warp) {
+  const int P = pp.npass, R0 = pp.radix[0], RL = pp.radix[P - 1];
+  if (P == 1) {
+    radix_dispatch(R0, [&](auto rc) {
+      pass_only<decltype(rc)::value, MAXE, true, Re>(pass_at<false>(pp, 0, 1, t, warp), in, out);
+    });
+    return;
+  }
+  radix_dispatch(RL, [&](auto rc) {
+    pass_head<decltype(rc)::value, MAXE, true>(pass_at<true>(pp, 0, 1, t, warp), x, in, true);
+  });
+  const int ns = middle_passes<MAXE, true, true>(pp, RL, t, x, twr, warp);
+  radix_dispatch(R0, [&](auto rc) {
+    pass_tail<decltype(rc)::value, MAXE, true>(pass_at<true>(pp, P - 1, ns, t, warp), x, twr, out, false);
+  });
+}
+
 // ---------------------------------------------------------------------------
 // plan policies: how the kernels below learn n, T and the radix passes.
 //   DynPlan   - runtime pass list (any 13-smooth length), radix by switch
@@ -871,19 +840,6 @@ struct DynPlan {
   __device__ __forceinline__ explicit DynPlan(const PassPlan& p) : pp(p) {}
   __device__ __forceinline__ int n() const { return pp.n; }
   __device__ __forceinline__ int T() const { return pp.T; }
-  // radix of the first executed pass (REV: passes run last-to-first)
-  template <bool REV, class F>
-  __device__ __forceinline__ void first(F&& f) const {
-    radix_dispatch(pp.radix[REV ? pp.npass - 1 : 0], f);
-  }
-  template <bool REV, class F>
-  __device__ __forceinline__ void last(F&& f) const {
-    radix_dispatch(pp.radix[REV ? 0 : pp.npass - 1], f);
-  }
-  template <bool INV, bool REV, class PL, class Re>
-  __device__ __forceinline__ void run(Cx<Re>* v, const PL& pl, Cx<Re>* sm, const Cx<Re>* tw) const {
-    run_passes<MAXE, INV>(v, pp, REV, pl, sm, tw, WarpLocal<PL>::value && warp_sized(pp.T));
-  }
   template <class Re, class PL>
   __device__ __forceinline__ Slots<Re, !PL::kLinear> slots(const PL& pl, Cx<Re>* sm) const {
     return Slots<Re, !PL::kLinear>{sm + pl.sidx(pp, 0), pl.pitch(pp), pl.pad(pp)};
@@ -896,6 +852,12 @@ struct DynPlan {
     const bool warp = WarpLocal<PL>::value && warp_sized(pp.T);
     if constexpr (kMerged) merged_transform<MAXE, INV>(pp, pl.t, slots<Re>(pl, sm), tw, in, out, SMIN, SMOUT, warp);
     else runtime_transform<MAXE, INV>(pp, pl.t, slots<Re>(pl, sm), tw, in, out, SMIN, SMOUT, warp);
+  }
+  template <class PL, class Re, class In, class Out>
+  __device__ __forceinline__ void inverse_reversed(const PL& pl, Cx<Re>* sm, const Cx<Re>* twr, const In& in,
+                                                   const Out& out) const {
+    runtime_inverse_reversed<MAXE>(pp, pl.t, slots<Re>(pl, sm), twr, in, out,
+                                   WarpLocal<PL>::value && warp_sized(pp.T));
   }
   template <class PL, class Re, class In, class Op, class Out>
   __device__ __forceinline__ void convolve(const PL& pl, Cx<Re>* sm, const Cx<Re>* tw, const Cx<Re>* twr,
@@ -943,6 +905,7 @@ struct FixPlan {
   __device__ __forceinline__ explicit FixPlan(const PassPlan& p) : pp(p) {}
   __device__ __forceinline__ static constexpr int n() { return N_; }
   __device__ __forceinline__ static constexpr int T() { return T_; }
+  // radix of the first executed pass (REV: passes run last-to-first)
   template <bool REV, class F>
   __device__ __forceinline__ void first(F&& f) const {
     f(IC<REV ? RLast<L>::value : RFirst<L>::value>{});
@@ -1167,14 +1130,52 @@ __global__ void __launch_bounds__(256, Plan::MAXE <= 8 ? 3 : 2) k_conv_pf(FftArg
   store_output<Plan, true, S, Re>(P, pl, a, v);
 }
 
+// The forward spectrum of a runtime plan's multi-kernel convolution, kept at
+// the points of its transform: the thread that stored a point reads it back.
+template <class Re>
+struct KeepOut {
+  Cx<Re>* p;  // point 0 of the thread's transform
+  int ps;     // slots between points
+  template <int R>
+  __device__ __forceinline__ void store(const Cx<Re>* v, int j, int nb) const {
+    Cx<Re>* q = p + j * ps;
+#pragma unroll
+    for (int r = 0; r < R; ++r, q += nb * ps) *q = v[r];
+  }
+};
+// the kept spectrum times (the conjugate of) one kernel
+template <class K, class Re, int KOP>
+struct KeepIn {
+  const Cx<Re>* p;
+  int ps;
+  const K* ker;
+  long long kps;
+  bool ok;
+  template <int R>
+  __device__ __forceinline__ void load(Cx<Re>* v, int j, int nb) const {
+    const Cx<Re>* q = p + j * ps;
+    const K* kq = ker + j * kps;
+    const long long step = nb * kps;
+#pragma unroll
+    for (int r = 0; r < R; ++r, q += nb * ps, kq += step) {
+      const Cx<Re> k = ok ? Conv<K, Re>::ld(kq) : mk<Re>(Re(0), Re(0));
+      v[r] = KOP == 0 ? cmulc(*q, k) : cmul(*q, k);
+    }
+  }
+};
+
 // Fused multi-kernel convolution (the reference's kernel_num > 1 shader,
 // vkdispatch/fft/shader_factories.py:166-193): the signal is read and
 // transformed once, then for each kernel k: * K_k (conjugate or plain
 // product) -> inverse FFT -> output slice k.  Kernel k is read at
 // a.ker + k * kstride and output slice k written at a.out + k * ostride
 // (elements).  The forward spectrum waits in a thread-private region at the
-// end of the dynamic shared memory (slot i * blockDim.x + threadIdx.x, MAXE
-// slots per thread), so only the exchange region is shared between threads.
+// end of the dynamic shared memory (MAXE slots per thread; a runtime plan keeps
+// point i of its transforms there, a compile-time plan value i of its thread),
+// so only the exchange region is shared between threads.  Runtime plans run the
+// self-contained passes, like every other transform (with values held in
+// registers across the passes, 3000 x 360 rows of three kernels took 43.2 us,
+// 31.4 here; 3000 x 1000 of four 110.8 and 81.1).
 template <class Plan, bool STRIDED, class S, class Re, int KOP>
 __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 32 ? 2 : 1)
     k_conv_multi(FftArgs a, int K, long long kstride, long long ostride) {
@@ -1188,39 +1189,50 @@ __global__ void __launch_bounds__(Plan::MAXE >= 32 ? 256 : 1024, Plan::MAXE >= 3
   unsigned dyn;
   asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
   Cx<Re>* keep = sm + (dyn / sizeof(Cx<Re>) - unsigned(MAXE) * blockDim.x);
-  Cx<Re> v[MAXE];
-  P.assume_t(pl.t);
-  const int n = P.n();
-  gather_input<Plan, S, Re>(P, pl, a, v);
   const bool kvalid = pl.tile_full || pl.valid;
-  P.template run<false, false>(v, pl, sm, tw);
-#pragma unroll
-  for (int i = 0; i < MAXE; ++i) keep[i * blockDim.x + threadIdx.x] = v[i];
-  for (int k = 0; k < K; ++k) {
-    if (k > 0) {
-#pragma unroll
-      for (int i = 0; i < MAXE; ++i) v[i] = keep[i * blockDim.x + threadIdx.x];
+  if constexpr (!IsFixPlan<Plan>::value) {
+    const int ps = STRIDED ? a.pp.M : 1;
+    Cx<Re>* kp = keep + (STRIDED ? pl.m : pl.m * P.n());
+    P.template transform<false, false, false>(pl, sm, tw, GlobalIn<S, Re>(a, pl, P.n()), KeepOut<Re>{kp, ps});
+    for (int k = 0; k < K; ++k) {
+      const S* ker = reinterpret_cast<const S*>(a.ker) + k * kstride + pl.ker0();
+      P.inverse_reversed(pl, sm, twr, KeepIn<S, Re, KOP>{kp, ps, ker, pl.ps, kvalid},
+                         GlobalOut<S, Re>(a, pl, reinterpret_cast<S*>(a.out) + k * ostride));
     }
-    const S* ker = reinterpret_cast<const S*>(a.ker) + k * kstride + pl.ker0();
-    P.template last<false>([&](auto rc) {
-      constexpr int RR = decltype(rc)::value;
-      constexpr int B = MAXE / RR;
-      const int nb = n / RR;
+  } else {
+    Cx<Re> v[MAXE];
+    P.assume_t(pl.t);
+    const int n = P.n();
+    gather_input<Plan, S, Re>(P, pl, a, v);
+    P.template run<false, false>(v, pl, sm, tw);
 #pragma unroll
-      for (int b = 0; b < B; ++b) {
-        const int j = pl.t + b * P.T();
-        if (j < nb) {
+    for (int i = 0; i < MAXE; ++i) keep[i * blockDim.x + threadIdx.x] = v[i];
+    for (int k = 0; k < K; ++k) {
+      if (k > 0) {
 #pragma unroll
-          for (int r = 0; r < RR; ++r) {
-            const int pos = j + r * nb;
-            const Cx<Re> kv = kvalid ? Conv<S, Re>::ld(ker + pos * pl.ps) : mk<Re>(Re(0), Re(0));
-            v[b * RR + r] = KOP == 0 ? cmulc(v[b * RR + r], kv) : cmul(v[b * RR + r], kv);
+        for (int i = 0; i < MAXE; ++i) v[i] = keep[i * blockDim.x + threadIdx.x];
+      }
+      const S* ker = reinterpret_cast<const S*>(a.ker) + k * kstride + pl.ker0();
+      P.template last<false>([&](auto rc) {
+        constexpr int RR = decltype(rc)::value;
+        constexpr int B = MAXE / RR;
+        const int nb = n / RR;
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+          const int j = pl.t + b * P.T();
+          if (j < nb) {
+#pragma unroll
+            for (int r = 0; r < RR; ++r) {
+              const int pos = j + r * nb;
+              const Cx<Re> kv = kvalid ? Conv<S, Re>::ld(ker + pos * pl.ps) : mk<Re>(Re(0), Re(0));
+              v[b * RR + r] = KOP == 0 ? cmulc(v[b * RR + r], kv) : cmul(v[b * RR + r], kv);
+            }
           }
         }
-      }
-    });
-    P.template run<true, true>(v, pl, sm, twr);
-    store_output<Plan, true, S, Re>(P, pl, a, v, reinterpret_cast<S*>(a.out) + k * ostride);
+      });
+      P.template run<true, true>(v, pl, sm, twr);
+      store_output<Plan, true, S, Re>(P, pl, a, v, reinterpret_cast<S*>(a.out) + k * ostride);
+    }
   }
 }
 

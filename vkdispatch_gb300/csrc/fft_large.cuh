@@ -9,7 +9,7 @@
 namespace vdx {
 
 // thread placement inside a column tile: m = column, t = thread of the column
-// (the interface run_passes / FixPlan::run use)
+// (the interface FixPlan::run uses)
 struct FsPlace {
   int t, m, M;
   static constexpr bool kLinear = true;
