@@ -95,12 +95,15 @@ __device__ __forceinline__ T block_reduce(T v, T* sh) {
 // blocks of 512 elements, 16 per lane of a warp.  Block k belongs to slot k % 8;
 // a lane folds the blocks of its slots, the slots are folded as a tree, and the
 // lanes last.  W warps (1 to 8) share a part's slots, and a CTA of eight warps
-// holds 8 / W parts.  That order depends on n alone, whatever W is, so results
-// do too, and W follows the amount of work: two warps per 4096 elements where
-// the parts fill the chip (one 512-thread CTA per part spent 16 instructions
-// per element, most of them on the fold: 1024 x 65536 floats took 54.9 us
-// against a copy rate of 39.5), eight where they do not (262144 complex
-// magnitudes on two warps a part took 11.4 us, their loads one after another).
+// holds 8 / W parts, numbered over all rows, so that short rows fill it too
+// (16384 x 4096 floats, one part a row: 81.6 us with a row's parts in a CTA of
+// their own, 45.7; 65000 x 512 97.2 and 43.7).  The order depends on n alone,
+// whatever W is, so results do too, and W follows the amount of work: two warps
+// per 4096 elements where the parts fill the chip (one 512-thread CTA per part
+// spent 16 instructions per element, most of them on the fold: 1024 x 65536
+// floats took 54.9 us against a copy rate of 39.5), eight where they do not
+// (262144 complex magnitudes on two warps a part took 11.4 us, their loads one
+// after another).
 //
 // A lane's elements of a block are neighbours in fours where n is a multiple of
 // four, in 16-byte loads if the part starts on such a boundary; rows of another
@@ -197,18 +200,19 @@ __device__ __forceinline__ T fold_block(const In* __restrict__ q, long long len,
 
 template <class In, class T, int OP, int MAP>
 __global__ void __launch_bounds__(32 * kWarps) k_reduce_partial(const In* __restrict__ in, long long n, long long chunk,
-                                                                T* __restrict__ part, int nparts, int W) {
+                                                                T* __restrict__ part, unsigned nparts, unsigned total,
+                                                                int W) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ T sh[kWarps][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w = warp & (W - 1);  // warp of its part; W is a power of two
-  const long long b = blockIdx.y;
-  const int p = blockIdx.x * (kWarps / W) + warp / W;
+  const unsigned g = blockIdx.x * unsigned(kWarps / W) + unsigned(warp / W);  // part, numbered over all rows
+  const unsigned b = g / nparts, p = g - b * nparts;
   const long long lo = (long long)p * chunk;
   const long long len = (lo + chunk < n ? lo + chunk : n) - lo;
   T acc = identity<T, OP>();
-  if (p < nparts && len > 0) {
-    const In* q = in + b * n + lo;
+  if (g < total && len > 0) {
+    const In* q = in + (long long)b * n + lo;
     const bool pack = n % kVec == 0;
     const bool vec = pack && reinterpret_cast<unsigned long long>(q) % alignof(Pack<In>) == 0;
     const int slots = kWarps / W;
@@ -240,7 +244,7 @@ __global__ void __launch_bounds__(32 * kWarps) k_reduce_partial(const In* __rest
   }
   if (w != 0) return;
   acc = warp_reduce<T, OP>(acc);
-  if (lane == 0 && p < nparts) part[b * nparts + p] = acc;
+  if (lane == 0 && g < total) part[g] = acc;
 }
 
 // Stage 2 folds the partials of a row in a fixed order: one warp per row for
@@ -271,11 +275,13 @@ template <class In, class T, int OP, int MAP>
 cudaError_t run(const void* in, long long n, long long batch, void* out, void* partials, int nparts, cudaStream_t s) {
   // parts start on 16-byte steps of the row
   const long long chunk = ((n + nparts - 1) / nparts + 3) & ~3ll;
-  const int W = part_warps(chunk, nparts * batch), G = kWarps / W;
-  const Launch l1{dim3((unsigned)((nparts + G - 1) / G), (unsigned)batch), dim3(32 * kWarps), 0, s};
+  const long long total = nparts * batch;  // at most 1024 parts of 65535 rows
+  const int W = part_warps(chunk, total), G = kWarps / W;
+  const Launch l1{dim3((unsigned)((total + G - 1) / G)), dim3(32 * kWarps), 0, s};
   const In* src = reinterpret_cast<const In*>(in);
   T* part = reinterpret_cast<T*>(partials);
-  cudaError_t e = enqueue(k_reduce_partial<In, T, OP, MAP>, l1, src, n, chunk, part, nparts, W);
+  cudaError_t e = enqueue(k_reduce_partial<In, T, OP, MAP>, l1, src, n, chunk, part, (unsigned)nparts,
+                          (unsigned)total, W);
   if (e != cudaSuccess) return e;
   Launch l2{dim3((unsigned)batch), dim3(kThreads), 0, s};
   if (nparts <= 32) {
