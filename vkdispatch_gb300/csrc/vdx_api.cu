@@ -1313,23 +1313,24 @@ TuneKey tune_key(int dev, const vdx_fft_desc& d, long long inner, long long oute
   const int N = (int)d.shape[d.axis];
   const int ib = inner == 1 ? 0 : 1 + std::min(floor_log2(inner), 20);
   return TuneKey{dev, d.kind, N, ib, std::min(floor_log2(outer), 24), d.io_type, d.compute_type, d.inverse,
-                 d.kernel_op, d.kernel_broadcast, d.flags & VDX_FFT_FLAG_TENSOR_CORE,
+                 d.kernel_op, d.kernel_broadcast,
+                 d.flags & (VDX_FFT_FLAG_TENSOR_CORE | VDX_FFT_FLAG_DENSE_REAL),
                  d.signal_lo < 0 && d.signal_hi < 0 ? 0 : 1};
 }
 
 // Median of 7 timed executions.  With `flush` (problems larger than a
 // quarter of L2) every execution starts from a cold L2, as it does when the
 // data streams through a long pipeline; smaller problems are timed warm.
-float time_plan(const vdx_plan* p, void* sig, const void* ker, cudaStream_t s, cudaEvent_t e0, cudaEvent_t e1,
-                void* flush, size_t flush_bytes) {
+float time_plan(const vdx_plan* p, void* in, void* out, const void* ker, cudaStream_t s, cudaEvent_t e0,
+                cudaEvent_t e1, void* flush, size_t flush_bytes) {
   for (int w = 0; w < 2; ++w)
-    if (vdx_fft_exec(p, sig, sig, ker, s) != VDX_OK) return -1.f;
+    if (vdx_fft_exec(p, in, out, ker, s) != VDX_OK) return -1.f;
   constexpr int reps = 7;
   float t[reps];
   for (int r = 0; r < reps; ++r) {
     if (flush) cudaMemsetAsync(flush, r, flush_bytes, s);
     cudaEventRecord(e0, s);
-    vdx_fft_exec(p, sig, sig, ker, s);
+    vdx_fft_exec(p, in, out, ker, s);
     cudaEventRecord(e1, s);
     if (cudaEventSynchronize(e1) != cudaSuccess) return -1.f;
     cudaEventElapsedTime(&t[r], e0, e1);
@@ -1384,7 +1385,6 @@ int autotune_plan(const vdx_fft_desc& d0, vdx_plan** plan) {
   }
   const long long outer_t = std::min(outer, std::max(1ll, cap / (long long)(row * inner_t * es)));
   vdx_fft_desc dt = d;
-  dt.flags &= ~VDX_FFT_FLAG_DENSE_REAL;  // the search runs in place on packed rows
   if (inner_t > 1) {
     dt.ndim = 3;
     dt.shape[0] = outer_t;
@@ -1399,7 +1399,10 @@ int autotune_plan(const vdx_fft_desc& d0, vdx_plan** plan) {
   const size_t sig_bytes = size_t(outer_t) * size_t(row) * size_t(inner_t) * es;
   const size_t ker_bytes = d.kind == VDX_KIND_CONV ? (d.kernel_broadcast ? size_t(row) * size_t(inner_t) * es : sig_bytes)
                                                     : 0;
+  // dense real rows run out of place, everything else in place
+  const bool dense = (d.flags & VDX_FFT_FLAG_DENSE_REAL) != 0;
   void* sig = nullptr;
+  void* dst = nullptr;
   void* ker = nullptr;
   void* flush = nullptr;
   int l2 = 0;
@@ -1408,6 +1411,7 @@ int autotune_plan(const vdx_fft_desc& d0, vdx_plan** plan) {
   cudaStream_t s = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   e = cudaMalloc(&sig, sig_bytes);
+  if (e == cudaSuccess && dense) e = cudaMalloc(&dst, sig_bytes);
   if (e == cudaSuccess && ker_bytes) e = cudaMalloc(&ker, ker_bytes);
   if (e == cudaSuccess) e = cudaMemset(sig, 0, sig_bytes);
   if (e == cudaSuccess && ker_bytes) e = cudaMemset(ker, 0, ker_bytes);
@@ -1436,9 +1440,10 @@ int autotune_plan(const vdx_fft_desc& d0, vdx_plan** plan) {
             t.fourstep = fsv;
             cands.push_back(t);
           }
-    // the 8-, 16- and 32-points-per-thread plans (16 differs from the
-    // default only where the default is 32: strided convolutions of 512 or
-    // 1024 points; create_plan refuses the combinations that have none)
+    // the 8-, 16- and 32-points-per-thread plans (16 differs from the default
+    // only where that is 32: strided transforms and convolutions of 512 or 1024
+    // points and 512-point convolutions along rows; create_plan refuses the
+    // combinations that have none)
     if (d.io_type == VDX_C64 && d.compute_type == VDX_C64)
       for (int pts : {8, 16, 32})
         for (int w : widths) {
@@ -1458,7 +1463,7 @@ int autotune_plan(const vdx_fft_desc& d0, vdx_plan** plan) {
         continue;
       }
       seen.emplace_back(sig_desc);
-      const float ms = time_plan(c, sig, ker, s, e0, e1, flush, flush_bytes);
+      const float ms = time_plan(c, sig, dense ? dst : sig, ker, s, e0, e1, flush, flush_bytes);
       ++tried;
       delete c;
       if (ms > 0.f && (best_ms < 0.f || ms < 0.97f * best_ms)) {
@@ -1471,6 +1476,7 @@ int autotune_plan(const vdx_fft_desc& d0, vdx_plan** plan) {
   if (e0) cudaEventDestroy(e0);
   if (s) cudaStreamDestroy(s);
   if (ker) cudaFree(ker);
+  if (dst) cudaFree(dst);
   if (sig) cudaFree(sig);
   if (flush) cudaFree(flush);
   cudaGetLastError();
