@@ -60,14 +60,13 @@ struct UnitPlan {
 };
 
 struct alignas(16) WorkUnit {
-  PassPlan pp;                  // the unit's pass plan (a copy, so one table read fetches everything)
+  PassPlan pp;                  // the unit's pass plan (a copy, so one read of the descriptor fetches everything)
   const Cx<float>* tw;          // stage-ordered twiddles of the unit's pass plan
   long long src, dst;           // element offset of point 0 of slot 0 (data or workspace)
   long long src_slot, dst_slot;  // elements between slots
   long long src_pt, dst_pt;     // elements between points
   const Cx<float>* twl;         // UK_COLS: W_L^{n2 k1} at k1 * L2 + n2
   int kind;
-  int plan;
   int nslots;  // slots (transforms, columns or rows) of this tile that exist
   int item;    // counter of a four-step item (UK_COLS signals it, UK_ROWS2 waits on it)
   int wait;    // UK_ROWS2: number of UK_COLS units of the item
@@ -78,7 +77,6 @@ struct alignas(16) WorkUnit {
 };
 
 struct BatchArgs {
-  const UnitPlan* plans;
   const WorkUnit* units;
   int nunits;
   int inverse;
@@ -344,7 +342,6 @@ struct vdx_batch_plan {
   size_t ws_bytes;
   size_t smem;
   int grid;
-  vdx::UnitPlan* d_plans;
   vdx::WorkUnit* d_units;
   unsigned* d_ticket;
   int* d_counters;
@@ -476,7 +473,6 @@ int vdx_batch_plan_create(const vdx_batch_item* items, int nitems, int inverse, 
       for (long long t0 = 0; t0 < it.count; t0 += M) {
         WorkUnit w{};
         w.kind = UK_ROWS;
-        w.plan = p;
         w.pp = plans[p].pp;
         w.tw = plans[p].tw;
         w.src = w.dst = it.offset + t0 * L;
@@ -513,7 +509,6 @@ int vdx_batch_plan_create(const vdx_batch_item* items, int nitems, int inverse, 
       for (int c0 = 0; c0 < L2; c0 += Mc) {
         WorkUnit w{};
         w.kind = UK_COLS;
-        w.plan = pc;
         w.pp = plans[pc].pp;
         w.tw = plans[pc].tw;
         w.src = it.offset + bt * L + c0;
@@ -533,7 +528,6 @@ int vdx_batch_plan_create(const vdx_batch_item* items, int nitems, int inverse, 
       for (int r0 = 0; r0 < L1; r0 += Mr) {
         WorkUnit w{};
         w.kind = UK_ROWS2;
-        w.plan = pr;
         w.pp = plans[pr].pp;
         w.tw = plans[pr].tw;
         w.src = wsoff + bt * L + (long long)r0 * L2;
@@ -576,18 +570,14 @@ int vdx_batch_plan_create(const vdx_batch_item* items, int nitems, int inverse, 
   p->smem = smem;
   p->grid = (nsm > 0 ? nsm : 148) * per_sm;
   p->cta = cta;
-  e = cudaMalloc(&p->d_plans, sizeof(UnitPlan) * plans.size());
-  if (e == cudaSuccess) e = cudaMalloc(&p->d_units, sizeof(WorkUnit) * units.size());
+  e = cudaMalloc(&p->d_units, sizeof(WorkUnit) * units.size());
   if (e == cudaSuccess) e = cudaMalloc(&p->d_ticket, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMalloc(&p->d_counters, sizeof(int) * std::max(1, nlarge));
   if (e == cudaSuccess) e = cudaMalloc(&p->d_status, sizeof(int));
   if (e == cudaSuccess)
-    e = cudaMemcpy(p->d_plans, plans.data(), sizeof(UnitPlan) * plans.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess)
     e = cudaMemcpy(p->d_units, units.data(), sizeof(WorkUnit) * units.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(p->d_status, 0, sizeof(int));
   if (e != cudaSuccess) {
-    cudaFree(p->d_plans);
     cudaFree(p->d_units);
     cudaFree(p->d_ticket);
     cudaFree(p->d_counters);
@@ -608,7 +598,6 @@ int vdx_batch_plan_create(const vdx_batch_item* items, int nitems, int inverse, 
 
 int vdx_batch_plan_destroy(vdx_batch_plan* p) {
   if (!p) return VDX_OK;
-  cudaFree(p->d_plans);
   cudaFree(p->d_units);
   cudaFree(p->d_ticket);
   cudaFree(p->d_counters);
@@ -641,7 +630,6 @@ int vdx_batch_exec(const vdx_batch_plan* p, void* data, void* workspace, void* s
     e = cudaMemsetAsync(p->d_counters, 0, sizeof(int) * p->nitems_large, s);
   if (e != cudaSuccess) return set_error(VDX_ERR_CUDA, cudaGetErrorString(e));
   BatchArgs a{};
-  a.plans = p->d_plans;
   a.units = p->d_units;
   a.nunits = p->nunits;
   a.inverse = p->inverse;

@@ -55,9 +55,10 @@ __global__ void k_conj_slab(Cx<Re>* K, const Cx<Re>* B, int M, long long inner) 
   K[e] = conj(B[e / inner]);
 }
 
-// ws (outer, M, inner) <- x (outer, N, inner) * w, zero-padded
-template <class S, class Re>
-__global__ void k_bs_in(const S* __restrict__ x, Cx<Re>* __restrict__ ws, const Cx<Re>* __restrict__ w,
+// The launches of convolutions longer than one CTA, which exist in fp32 compute
+// only.  ws (outer, M, inner) <- x (outer, N, inner) * w, zero-padded
+template <class S>
+__global__ void k_bs_in(const S* __restrict__ x, Cx<float>* __restrict__ ws, const Cx<float>* __restrict__ w,
                         long long outer, int N, int M, long long inner) {
   const long long total = outer * M * inner;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
@@ -66,16 +67,16 @@ __global__ void k_bs_in(const S* __restrict__ x, Cx<Re>* __restrict__ ws, const 
     const long long om = e / inner;
     const int m = int(om % M);
     const long long o = om / M;
-    Cx<Re> v = mk<Re>(Re(0), Re(0));
-    if (m < N) v = cmul(Conv<S, Re>::ld(x + (o * N + m) * inner + i), ldg(w + m));
+    Cx<float> v = mk<float>(0.f, 0.f);
+    if (m < N) v = cmul(Conv<S, float>::ld(x + (o * N + m) * inner + i), ldg(w + m));
     ws[e] = v;
   }
 }
 
 // y (outer, N, inner) <- ws[:, :N, :] * w * scale
-template <class S, class Re>
-__global__ void k_bs_out(const Cx<Re>* __restrict__ ws, S* __restrict__ y, const Cx<Re>* __restrict__ w,
-                         long long outer, int N, int M, long long inner, Re sc) {
+template <class S>
+__global__ void k_bs_out(const Cx<float>* __restrict__ ws, S* __restrict__ y, const Cx<float>* __restrict__ w,
+                         long long outer, int N, int M, long long inner, float sc) {
   const long long total = outer * N * inner;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
@@ -83,15 +84,14 @@ __global__ void k_bs_out(const Cx<Re>* __restrict__ ws, S* __restrict__ y, const
     const long long ok = e / inner;
     const int k = int(ok % N);
     const long long o = ok / N;
-    const Cx<Re> v = ws[(o * M + k) * inner + i];
-    Conv<S, Re>::st(y + e, scale(cmul(v, ldg(w + k)), sc));
+    const Cx<float> v = ws[(o * M + k) * inner + i];
+    Conv<S, float>::st(y + e, scale(cmul(v, ldg(w + k)), sc));
   }
 }
 
 // ws (outer, M, inner) *= conj(K[m][i]): the spectrum product of the long
 // (four-step) form, where the convolution is two separate transforms
-template <class Re>
-__global__ void k_bs_mul(Cx<Re>* __restrict__ ws, const Cx<Re>* __restrict__ K, long long outer, long long slab) {
+__global__ void k_bs_mul(Cx<float>* __restrict__ ws, const Cx<float>* __restrict__ K, long long outer, long long slab) {
   const long long total = outer * slab;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x)
@@ -103,17 +103,17 @@ unsigned grid_for(long long total, int threads) {
   return (unsigned)std::min<long long>(std::max<long long>(g, 1), 152 * 32);
 }
 
-template <class S, class Re>
+template <class S>
 cudaError_t launch_io(bool in_phase, const void* x, void* ws, const void* w, long long outer, int N, int M,
-                      long long inner, double scale, cudaStream_t s) {
+                      long long inner, float scale, cudaStream_t s) {
   constexpr int TH = 256;
   if (in_phase) {
-    k_bs_in<S, Re><<<grid_for(outer * M * inner, TH), TH, 0, s>>>(
-        static_cast<const S*>(x), static_cast<Cx<Re>*>(ws), static_cast<const Cx<Re>*>(w), outer, N, M, inner);
+    k_bs_in<S><<<grid_for(outer * M * inner, TH), TH, 0, s>>>(static_cast<const S*>(x), static_cast<Cx<float>*>(ws),
+                                                             static_cast<const Cx<float>*>(w), outer, N, M, inner);
   } else {
-    k_bs_out<S, Re><<<grid_for(outer * N * inner, TH), TH, 0, s>>>(
-        static_cast<const Cx<Re>*>(ws), static_cast<S*>(const_cast<void*>(x)), static_cast<const Cx<Re>*>(w), outer,
-        N, M, inner, Re(scale));
+    k_bs_out<S><<<grid_for(outer * N * inner, TH), TH, 0, s>>>(
+        static_cast<const Cx<float>*>(ws), static_cast<S*>(const_cast<void*>(x)), static_cast<const Cx<float>*>(w),
+        outer, N, M, inner, scale);
   }
   return cudaGetLastError();
 }
@@ -141,23 +141,20 @@ cudaError_t launch_conj_slab(void* K, const void* B, int M, long long inner, boo
   return cudaGetLastError();
 }
 
-cudaError_t launch_bluestein_mul(void* ws, const void* K, long long outer, int M, long long inner, bool f64,
-                                 cudaStream_t s) {
+cudaError_t launch_bluestein_mul(void* ws, const void* K, long long outer, int M, long long inner, cudaStream_t s) {
   constexpr int TH = 256;
   const long long slab = (long long)M * inner;
   const unsigned g = grid_for(outer * slab, TH);
-  if (f64) k_bs_mul<double><<<g, TH, 0, s>>>(static_cast<Cx<double>*>(ws), static_cast<const Cx<double>*>(K), outer, slab);
-  else k_bs_mul<float><<<g, TH, 0, s>>>(static_cast<Cx<float>*>(ws), static_cast<const Cx<float>*>(K), outer, slab);
+  k_bs_mul<<<g, TH, 0, s>>>(static_cast<Cx<float>*>(ws), static_cast<const Cx<float>*>(K), outer, slab);
   return cudaGetLastError();
 }
 
 cudaError_t launch_bluestein_io(bool in_phase, int store, const void* x, void* ws, const void* w, long long outer,
-                                int N, int M, long long inner, double scale, cudaStream_t s) {
+                                int N, int M, long long inner, float scale, cudaStream_t s) {
   switch (store) {
-    case ST_C64: return launch_io<Cx<float>, float>(in_phase, x, ws, w, outer, N, M, inner, scale, s);
-    case ST_C32: return launch_io<c32s, float>(in_phase, x, ws, w, outer, N, M, inner, scale, s);
-    case ST_BF16: return launch_io<bf16c, float>(in_phase, x, ws, w, outer, N, M, inner, scale, s);
-    case ST_C128: return launch_io<Cx<double>, double>(in_phase, x, ws, w, outer, N, M, inner, scale, s);
+    case ST_C64: return launch_io<Cx<float>>(in_phase, x, ws, w, outer, N, M, inner, scale, s);
+    case ST_C32: return launch_io<c32s>(in_phase, x, ws, w, outer, N, M, inner, scale, s);
+    case ST_BF16: return launch_io<bf16c>(in_phase, x, ws, w, outer, N, M, inner, scale, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -21,7 +21,7 @@ __global__ void k_cross_twiddle(Cx<float>* tab, int N1, int N0) {
   if (i >= N1 * N0) return;
   const int k1 = i / N0, b0 = i - k1 * N0;
   double s, c;
-  sincospi(2.0 * double(b0 * k1) / double(N1 * N0), &s, &c);  // b0 k1 < N1 N0 <= 2^24
+  sincospi(2.0 * double(b0 * k1) / double(N1 * N0), &s, &c);  // b0 k1 < N1 N0 <= 2^28
   tab[i] = mk<float>(float(c), float(-s));
 }
 

@@ -674,13 +674,10 @@ int plan_fourstep(vdx_plan* p, long long inner, long long outer, int smem_optin)
     p->ws = nullptr;
     return fail(VDX_ERR_NOMEM, std::string("four-step workspace: ") + cudaGetErrorString(e));
   }
-  e = cudaMalloc(reinterpret_cast<void**>(&p->d_status), sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(p->d_status, 0, sizeof(int));
-  if (e != cudaSuccess) {
-    p->d_status = nullptr;
-    return cuda_fail(e, "four-step status word");
-  }
   if (p->tensor_core) {
+    e = cudaMalloc(reinterpret_cast<void**>(&p->d_status), sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(p->d_status, 0, sizeof(int));
+    if (e != cudaSuccess) return cuda_fail(e, "four-step status word");
     // 128-point tiles of 16 (8-byte) or 32 (4-byte) columns, 128 threads
     if (N1 != 128 || N0 != 128 || ppA.M != ppB.M || (ppA.M != 16 && ppA.M != 32))
       return fail(VDX_ERR_UNSUPPORTED, "tensor-core stages need 128 x 128 tiles of 16 or 32 columns");
@@ -1728,16 +1725,16 @@ int exec_plan(const vdx_plan* p, const void* in, void* out, const void* kernel, 
       if (e != cudaSuccess) return cuda_fail(e, "Bluestein launch");
       return VDX_OK;
     }
-    e = launch_bluestein_io(true, p->store, in, p->bs_ws, p->bs_w, p->outer, p->N, p->bs_M, p->inner, 1.0, s);
+    e = launch_bluestein_io(true, p->store, in, p->bs_ws, p->bs_w, p->outer, p->N, p->bs_M, p->inner, 1.f, s);
     if (e != cudaSuccess) return cuda_fail(e, "Bluestein chirp-in launch");
     int rc = exec_plan(p->bs_fwd, p->bs_ws, p->bs_ws, nullptr, nullptr, stream);
     if (rc != VDX_OK) return rc;
-    e = launch_bluestein_mul(p->bs_ws, p->bs_K, p->outer, p->bs_M, p->inner, p->f64, s);
+    e = launch_bluestein_mul(p->bs_ws, p->bs_K, p->outer, p->bs_M, p->inner, s);
     if (e != cudaSuccess) return cuda_fail(e, "Bluestein spectrum product launch");
     rc = exec_plan(p->bs_inv, p->bs_ws, p->bs_ws, nullptr, nullptr, stream);
     if (rc != VDX_OK) return rc;
     e = launch_bluestein_io(false, p->store, out, p->bs_ws, p->bs_w, p->outer, p->N, p->bs_M, p->inner,
-                            norm_scale(p->d.normalize, p->N), s);
+                            float(norm_scale(p->d.normalize, p->N)), s);
     if (e != cudaSuccess) return cuda_fail(e, "Bluestein chirp-out launch");
     return VDX_OK;
   }
