@@ -50,6 +50,10 @@ cudaError_t launch_conv_layout(const FftArgs& a, const Launch& l, int variant) {
     // axis 1: 74.1 -> 48.8), wrong for one that all share and L2 should keep
     // (40 x 1024 x 256: 75.8 -> 81.9), and at 1024 points wrong where the forward
     // spectrum is written too (64 x 1024 x 33: 24.2 -> 45.5).
+    // Plans of up to 16 points gain by the early loads either way and read every
+    // spectrum evict-first: for shared ones that costs 0 to 5 % (65536 x 256 rows
+    // 48.0 us, 45.5 with plain loads; 16384 x 1024 66.0 and 65.4), and choosing the
+    // policy at run time costs own ones as much (16384 x 1024 70.4 -> 73.6).
     const bool early = Plan::MAXE <= 16 || (a.ker_bs != 0 && (variant == 0 || a.pp.n < 1024));
     if (l.block.x <= 256 && early && conv_prefetch()) {
       if (variant == 0) return enqueue_pdl(k_conv_pf<Plan, STRIDED, S, Re, KOP>, l, a);

@@ -2,12 +2,11 @@
 //
 // Same two-stage shape as the reference (vkdispatch/reduce/stage.py:31-145:
 // grid-stride accumulate -> shared-memory tree -> subgroup butterfly; stage 2
-// folds the per-workgroup partials), re-designed: each CTA owns one
-// contiguous chunk of a row and keeps four independent loads in flight per
-// thread, the tree is warp shuffles plus one 32-slot shared array, partials
-// go to a caller-provided workspace rather than the output buffer, and stage
-// 2 folds the partials of a row in a fixed order, so results depend only on
-// n and never on scheduling.
+// folds the per-workgroup partials), re-designed: one to eight warps fold a
+// part of a row, loads of a whole block in flight, a tree of slots and lanes
+// whose order depends on n alone; partials go to a caller-provided workspace
+// rather than the output buffer, and stage 2 folds the partials of a row in a
+// fixed order, so results never depend on scheduling.
 #include "vdx_internal.h"
 #include "vdx.h"
 

@@ -7,10 +7,11 @@
 //   };
 // io is the reference's mapped_io_index() (the element's flat index in the
 // buffer: row * n + i), and the map may read any of the call's buffers and
-// scalars through m.  The two stages have the shape of the ahead-of-time
-// kernels of reduce.cu: each CTA folds one contiguous chunk of a row with
-// four independent maps in flight per thread, warp shuffles and one 32-slot
-// shared array; stage 2 folds a row's partials in a fixed order.
+// scalars through m.  Stage 1 is of its own form, not that of reduce.cu: each
+// 512-thread CTA folds one contiguous chunk of a row with four independent maps
+// in flight per thread (a map may cost anything, so a part is not sized by its
+// bytes), warp shuffles and one 32-slot shared array; stage 2 folds a row's
+// partials in a fixed order.
 #pragma once
 
 #include "fft_mapped.cuh"

@@ -297,9 +297,10 @@ class ReduceFunction:
                 compiled = True
         if not compiled:
             s1 = (f"// stage 1: vdx::k_reduce_partial<In, T, {name}, {maps}> of libvdx.so (sm_103a):\n"
-                  "// grid (parts, rows) x 512 threads; each CTA folds one contiguous chunk of a row")
-            s2 = (f"// stage 2: vdx::k_reduce_final<T, {name}>: one CTA per row folds its partials in a fixed "
-                  "order")
+                  "// CTAs of eight warps; one to eight warps fold a part (4096 or more elements of a row)\n"
+                  "// in an order that depends on the row length alone, and a CTA holds parts of any rows")
+            s2 = (f"// stage 2: vdx::k_reduce_final<T, {name}>: one warp per row folds up to 32 partials in a\n"
+                  "// fixed order (CTAs of one or four warps), one 512-thread CTA per row folds more")
         else:
             args = [0.0 if sc else _Placeholder(t) for t, sc in zip(self.map_func.input_dtypes(),
                                                                     self.map_func.arg_is_scalar())]
@@ -309,7 +310,7 @@ class ReduceFunction:
             s1 = ("// stage 1, compiled with NVRTC (csrc/reduce_mapped.cuh)\n" + hooks +
                   f"// vdx::reduce_mapped_partial<VdxReduceHooks, Re, {acc}, {name}>")
             s2 = f"// stage 2: vdx::reduce_mapped_final<{acc}, {name}>"
-        return [ShaderSource("reduction stage 1", _numbered(s1, bool(line_numbers)), (512, 1, 1)),
+        return [ShaderSource("reduction stage 1", _numbered(s1, bool(line_numbers)), (512 if compiled else 256, 1, 1)),
                 ShaderSource("reduction stage 2", _numbered(s2, bool(line_numbers)), (512, 1, 1))]
 
     def print_src(self, line_numbers: bool = None):
