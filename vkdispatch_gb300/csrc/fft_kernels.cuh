@@ -1116,13 +1116,15 @@ __global__ void __launch_bounds__(256, Plan::MAXE <= 8 ? 3 : 2) k_conv_pf(FftArg
     });
   }
   Plan::template each<RR>(pl.t, [&](auto b, int j) {
-    // no stepping pointer: 32 addresses in a chain keep the loads from going out
-    // together (64 x 1024 x 512 along axis 1: 260.8 -> 181.7 us)
+    const S* q = ker + j * pl.ps;
 #pragma unroll
-    for (int r = 0; r < RR; ++r) {
+    for (int r = 0; r < RR; ++r, q += step) {
       Cx<Re> k;
+      // 32 points: no stepping pointer, since a chain of 32 addresses keeps the
+      // loads from going out together (64 x 1024 x 512 along axis 1: 260.8 ->
+      // 181.7 us; chains of 16 do as well: 64 x 512 x 257 43.4 and 43.7)
       if constexpr (PF) k = kr[b * RR + r];
-      else k = kvalid ? ld_once<S, Re>(ker + (j + r * nb) * pl.ps) : mk<Re>(Re(0), Re(0));
+      else k = kvalid ? ld_once<S, Re>(RR >= 32 ? ker + (j + r * nb) * pl.ps : q) : mk<Re>(Re(0), Re(0));
       v[b * RR + r] = KOP == 0 ? cmulc(v[b * RR + r], k) : cmul(v[b * RR + r], k);
     }
   });
