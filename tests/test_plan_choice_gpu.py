@@ -1,6 +1,7 @@
 """Choices of the planner for runtime lengths, and the kernels on them: in lists
 of even radices the pass whose scatter conflicts least runs first; rows of 33 to
-48 threads share a CTA where they are short."""
+48 threads share a CTA where they are short; long columns of many transforms keep
+to 512 threads."""
 
 import numpy as np
 import pytest
@@ -65,3 +66,17 @@ def test_rows_per_cta(n, rows_per_cta):
     rb = vd.asrfftbuffer(r)
     vd.fft.rfft(rb)
     assert rel_l2(rb.read_fourier(0), np.fft.rfft(r.astype(np.float64), axis=-1)) <= tol_fp32(2 * n)
+
+
+@pytest.mark.parametrize("n,wide", [(5200, 520), (5600, 560), (6400, 640), (6000, 600)])
+def test_columns_per_tile(n, wide):
+    rng = np.random.default_rng(n)
+    for inner, threads in ((5, wide), (400, 512)):
+        d = _plan((1, n, inner))
+        assert d["threads_per_transform"] <= threads
+        x = crandn(rng, (1, n, inner))
+        b = vd.asbuffer(x)
+        vd.fft.fft(b, axis=1)
+        assert rel_l2(b.read(0), np.fft.fft(x.astype(np.complex128), axis=1)) <= tol_fp32(n)
+        vd.fft.ifft(b, axis=1)
+        assert rel_l2(b.read(0), x) <= 2 * tol_fp32(n)

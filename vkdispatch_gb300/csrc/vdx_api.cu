@@ -1076,6 +1076,20 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
       return plan_bluestein(d, inner, outer, N, st, f64, plan);
     return fail(VDX_ERR_UNSUPPORTED, why + " (VDX_FFT_FLAG_BLUESTEIN plans such lengths)");
   }
+  // a column of more than 512 threads leaves its tile one column, 8 bytes of every
+  // 32-byte sector: the cheapest list of up to 512 threads runs instead where it
+  // has no more passes (50 x 5200 x 32: 134.6 us as 13 x 10 x 10 x 4, 91.6 as 13 x
+  // 16 x 5 x 5; 3 x 5600 x 512 and its like 1.13 times as fast; with a pass more a
+  // quarter of the shapes lose).  Up to one column per SM the narrow tile wins, as
+  // it has the more CTAs (1 x 6000 x 32: 14.4 and 17.5 us)
+  if (inner > 1 && maxe == 16 && pmaxe == 16 && threads_of(n, p->radices) > 512) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->dev);
+    std::vector<int> r;
+    if (outer * inner > sms && factor_radices(n, maxe, r, why, 512) && r.size() <= p->radices.size() &&
+        threads_of(n, r) <= 512)
+      p->radices = r;
+  }
   if (tune.order == 1) std::reverse(p->radices.begin(), p->radices.end());
   if (pmaxe == 32) p->radices = {32, n / 32};  // the two-pass compile-time plan
 
