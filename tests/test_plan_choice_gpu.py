@@ -1,7 +1,7 @@
 """Choices of the planner for runtime lengths, and the kernels on them: in lists
 of even radices the pass whose scatter conflicts least runs first; rows of 33 to
 48 threads share a CTA where they are short; long columns of many transforms keep
-to 512 threads."""
+to 512 threads; tiles of 3, 5, 6 or 7 columns give way to 2 or 4."""
 
 import numpy as np
 import pytest
@@ -80,3 +80,20 @@ def test_columns_per_tile(n, wide):
         assert rel_l2(b.read(0), np.fft.fft(x.astype(np.complex128), axis=1)) <= tol_fp32(n)
         vd.fft.ifft(b, axis=1)
         assert rel_l2(b.read(0), x) <= 2 * tol_fp32(n)
+
+
+@pytest.mark.parametrize("n", [1500, 2000, 2100, 2205, 4095])
+@pytest.mark.parametrize("inner", [1, 3, 33, 700])
+def test_column_tiles(n, inner):
+    rng = np.random.default_rng(n + inner)
+    x = crandn(rng, (1, n, inner))
+    if inner == 33:  # fewer tiles than SMs, whatever their width
+        assert _plan((1, n, inner))["transforms_per_cta"] in (2, 4, 8)
+    b = vd.asbuffer(x)
+    vd.fft.fft(b, axis=1)
+    assert rel_l2(b.read(0), np.fft.fft(x.astype(np.complex128), axis=1)) <= tol_fp32(n)
+    k = crandn(rng, (1, n, inner))
+    c = vd.asbuffer(x)
+    vd.fft.convolve(c, vd.asbuffer(k), axis=1)
+    want = np.fft.ifft(np.fft.fft(x.astype(np.complex128), axis=1) * np.conj(k), axis=1)
+    assert rel_l2(c.read(0), want) <= 2 * tol_fp32(n)

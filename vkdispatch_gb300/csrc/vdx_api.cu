@@ -1156,10 +1156,25 @@ int create_plan(const vdx_fft_desc* desc, const Tune& tune, vdx_plan** plan) {
     // 1024 x 96 x 170: 57.9, 52.5, 57.3; but 64 x 512 x 512: 55.7, 62.9, 71.3
     // and 16 x 1024 x 1024: 69.2, 76.3)
     int mcols = !f64 && pmaxe == 16 && T <= 16 ? 16 : 8;
-    if (const char* e = std::getenv("VDX_STRIDED_COLUMNS")) mcols = std::max(1, std::min(32, std::atoi(e)));
+    const char* env = std::getenv("VDX_STRIDED_COLUMNS");
+    const bool asked = env || tune.width > 0;
+    if (env) mcols = std::max(1, std::min(32, std::atoi(env)));
     if (tune.width > 0) mcols = std::min(32, tune.width);
     M = (int)std::min<long long>(mcols, inner);
     M = std::max(1, std::min(M, (pmaxe == 32 ? 256 : 1024) / T));  // 32-point plans: CTAs of <= 256 threads
+    // Where the threads leave 3, 5, 6 or 7 columns, the power of two below while
+    // every narrower tile has an SM of its own, so that a launch of one wave does
+    // less per CTA (56 lengths of 3 columns, 300 columns in all 1.26; many columns
+    // 0.92); and for 5, whose 40-byte rows touch two sectors of which four columns
+    // fill one, in larger launches too (33 lengths, each size 1.09 to 1.31 times as
+    // fast), unless that makes two waves of one (20 x 1638 x 32: 0.78)
+    if (!asked && !f64 && pmaxe == 16 && M == 1024 / T && M > 2 && M < 8 && M != 4) {
+      const int m = M == 3 ? 2 : 4;
+      const long long wide = outer * ((inner + M - 1) / M), narrow = outer * ((inner + m - 1) / m);
+      int sms = 0;
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->dev);
+      if (narrow <= sms || (M == 5 && wide > sms)) M = m;
+    }
     while (M > 1 && need_smem && size_t(n) * M * cbytes > size_t(smem_optin)) M /= 2;
     smem = need_smem ? size_t(n) * M * cbytes : 0;
   } else {
