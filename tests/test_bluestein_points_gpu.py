@@ -44,3 +44,12 @@ def test_half_storage(choice, n, storage, tol):
 def test_c64(choice, n):
     # forward and inverse convolutions of the chirp at up to 4n points
     _check(n, vd.complex64, 3 * tol_fp32(4 * n))
+
+
+@pytest.mark.parametrize("storage,tol", [(vd.complex32, 2.5e-3), (vd.complexbf16, 1.6e-2), (vd.complex128, 1e-12)])
+@pytest.mark.parametrize("n", [211, 2053, 4093])
+def test_default_plans(n, storage, tol):
+    """M = 512, whose rows default to the two-pass plan on complex64, and 8192,
+    the longest convolution of fp64."""
+    P.cache_clear()
+    _check(n, storage, tol)
