@@ -125,10 +125,20 @@ cudaError_t launch_dyn_conv_layout(const FftArgs& a, const Launch& l, int kop, i
 template <class S, class Re>
 cudaError_t launch_dyn_real(const FftArgs& a, const Launch& l, int op);
 
+// fp64 Bluestein transforms are bound by the few fp64 units of an SM, so the
+// CTAs' spread over the SMs counts: a launch that starts while another drains
+// (enqueue_pdl) finds some SMs fuller than others and keeps that imbalance (one
+// after another, 500 x 509: 152.3 us, 94.3 with plain launches; 4000 x 121 146.2
+// and 131.1, 300 x 1009 145.8 and 101.4).
 template <class Plan, class S, class Re>
 cudaError_t launch_bluestein(const FftArgs& a, const Launch& l, bool strided) {
-  if (strided) return enqueue_pdl(k_bluestein<Plan, true, S, Re>, l, a);
-  return enqueue_pdl(k_bluestein<Plan, false, S, Re>, l, a);
+  if constexpr (Same<Re, double>::value) {
+    if (strided) return enqueue(k_bluestein<Plan, true, S, Re>, l, a);
+    return enqueue(k_bluestein<Plan, false, S, Re>, l, a);
+  } else {
+    if (strided) return enqueue_pdl(k_bluestein<Plan, true, S, Re>, l, a);
+    return enqueue_pdl(k_bluestein<Plan, false, S, Re>, l, a);
+  }
 }
 template <class S, class Re>
 cudaError_t launch_dyn_bluestein(const FftArgs& a, const Launch& l, bool strided);
