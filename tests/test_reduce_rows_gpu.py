@@ -29,9 +29,11 @@ def _rows(fn, t, vt):
 
 
 # (rows, n): 64 elements, a whole block, one part of two warps, of one warp by
-# its number, two parts, and 16 parts of two warps; n odd where rows misalign
+# its number, two parts, and 16 parts of two warps; n odd where rows misalign.
+# The last: rows that leave places of a CTA empty (5 and 18 parts in fours) and
+# that do not
 SHAPES = [(16384, 64), (20001, 65), (9000, 512), (4097, 2048), (5000, 1023), (6001, 4096), (2501, 4099), (333, 8191),
-          (1024, 65536)]
+          (1024, 65536), (1500, 18001), (400, 70000), (148, 21716), (33, 100001)]
 
 
 @pytest.mark.parametrize("rows,n", SHAPES)

@@ -94,15 +94,16 @@ __device__ __forceinline__ T block_reduce(T v, T* sh) {
 // blocks of 512 elements, 16 per lane of a warp.  Block k belongs to slot k % 8;
 // a lane folds the blocks of its slots, the slots are folded as a tree, and the
 // lanes last.  W warps (1 to 8) share a part's slots, and a CTA of eight warps
-// holds 8 / W parts, numbered over all rows, so that short rows fill it too
-// (16384 x 4096 floats, one part a row: 81.6 us with a row's parts in a CTA of
-// their own, 45.7; 65000 x 512 97.2 and 43.7).  The order depends on n alone,
-// whatever W is, so results do too, and W follows the amount of work: two warps
-// per 4096 elements where the parts fill the chip (one 512-thread CTA per part
-// spent 16 instructions per element, most of them on the fold: 1024 x 65536
-// floats took 54.9 us against a copy rate of 39.5), eight where they do not
-// (262144 complex magnitudes on two warps a part took 11.4 us, their loads one
-// after another).
+// holds 8 / W parts: of its row, or, where more than one in 16 would stay empty
+// that way, numbered over all rows (16384 x 4096 floats, one part a row: 81.6 us
+// by rows, 45.3; 65000 x 512 97.2 and 43.3; 20000 x 18000 complex, five parts,
+// 457 and 414; but 148 x 21716 complex, no place empty, 8.3 by rows and 9.2 over
+// all).  The order depends on n alone, whatever W is, so results do too, and W
+// follows the amount of work: two warps per 4096 elements where the parts fill
+// the chip (one 512-thread CTA per part spent 16 instructions per element, most
+// of them on the fold: 1024 x 65536 floats took 54.9 us against a copy rate of
+// 39.5), eight where they do not (262144 complex magnitudes on two warps a part
+// took 11.4 us, their loads one after another).
 //
 // A lane's elements of a block are neighbours in fours where n is a multiple of
 // four, in 16-byte loads if the part starts on such a boundary; rows of another
@@ -205,12 +206,24 @@ __global__ void __launch_bounds__(32 * kWarps) k_reduce_partial(const In* __rest
   __shared__ T sh[kWarps][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w = warp & (W - 1);  // warp of its part; W is a power of two
-  const unsigned g = blockIdx.x * unsigned(kWarps / W) + unsigned(warp / W);  // part, numbered over all rows
-  const unsigned b = g / nparts, p = g - b * nparts;
+  const unsigned u = blockIdx.x * unsigned(kWarps / W) + unsigned(warp / W);
+  unsigned b, p, g;
+  bool live;
+  if (total) {  // parts numbered over all rows
+    g = u;
+    b = g / nparts;
+    p = g - b * nparts;
+    live = g < total;
+  } else {
+    b = blockIdx.y;
+    p = u;
+    g = b * nparts + p;
+    live = p < nparts;
+  }
   const long long lo = (long long)p * chunk;
   const long long len = (lo + chunk < n ? lo + chunk : n) - lo;
   T acc = identity<T, OP>();
-  if (g < total && len > 0) {
+  if (live && len > 0) {
     const In* q = in + (long long)b * n + lo;
     const bool pack = n % kVec == 0;
     const bool vec = pack && reinterpret_cast<unsigned long long>(q) % alignof(Pack<In>) == 0;
@@ -243,7 +256,7 @@ __global__ void __launch_bounds__(32 * kWarps) k_reduce_partial(const In* __rest
   }
   if (w != 0) return;
   acc = warp_reduce<T, OP>(acc);
-  if (lane == 0 && g < total) part[g] = acc;
+  if (lane == 0 && live) part[g] = acc;
 }
 
 // Stage 2 folds the partials of a row in a fixed order: one warp per row for
@@ -276,11 +289,14 @@ cudaError_t run(const void* in, long long n, long long batch, void* out, void* p
   const long long chunk = ((n + nparts - 1) / nparts + 3) & ~3ll;
   const long long total = nparts * batch;  // at most 1024 parts of 65535 rows
   const int W = part_warps(chunk, total), G = kWarps / W;
-  const Launch l1{dim3((unsigned)((total + G - 1) / G)), dim3(32 * kWarps), 0, s};
+  const int per_row = (nparts + G - 1) / G;
+  const bool flat = (per_row * G - nparts) * 16 > nparts;
+  const dim3 grid = flat ? dim3((unsigned)((total + G - 1) / G)) : dim3((unsigned)per_row, (unsigned)batch);
+  const Launch l1{grid, dim3(32 * kWarps), 0, s};
   const In* src = reinterpret_cast<const In*>(in);
   T* part = reinterpret_cast<T*>(partials);
   cudaError_t e = enqueue(k_reduce_partial<In, T, OP, MAP>, l1, src, n, chunk, part, (unsigned)nparts,
-                          (unsigned)total, W);
+                          flat ? (unsigned)total : 0u, W);
   if (e != cudaSuccess) return e;
   Launch l2{dim3((unsigned)batch), dim3(kThreads), 0, s};
   if (nparts <= 32) {
